@@ -206,8 +206,7 @@ void Engine::launch(int id, bool rev) {
         runMpk(*this, *f.mpk, f.ops, f.power);
         lastStatus = f.mpk->status.p;
     } else {
-        runSweep(*this, f, rev);
-        lastStatus = dStatus.p;
+        runSweep(*this, f, rev);  // sets lastStatus
     }
 }
 

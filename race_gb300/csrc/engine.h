@@ -135,7 +135,8 @@ struct DevWaves {
     // order: the rows of a wave sorted by length, cut into chunks of 32
     // positions; each position's entries in groups of four slots (entry k
     // of chunk lane l at off + 32 (k - k % 4) + 4 l + k % 4). Per wave its
-    // first chunk (numWaves+1), per chunk its first slot.
+    // first chunk (numWaves+1), per chunk its first slot. Where the dataflow
+    // executor runs a Gauss-Seidel function, sellCol holds its marked columns.
     bool sell = false;
     int sellMidRow = 0;
     long long sellSlots = 0;
@@ -143,6 +144,19 @@ struct DevWaves {
     DevBuf<long long> chunkOff;
     DevBuf<unsigned char> sellVal;  // sellSlots values (the operands' value type)
     DevBuf<int> sellCol;
+};
+
+// Task lists of the dataflow executor (flow.cu) for one direction of a
+// Gauss-Seidel or Kaczmarz function, with the wave executor's sums (0) and
+// the leaf executor's (1).
+struct DevFlow {
+    bool ok = false;            // FlowOrder::ok (waves.h)
+    int numTasks[2] = {0, 0};
+    DevBuf<int4> task[2];
+    DevBuf<int4> pos;           // per wave plan position: row, first entry, length
+    DevBuf<int> mark;           // per matrix entry (FlowArgs::mark)
+    DevBuf<int> sellMark;       // Kaczmarz: the marks in the order of DevWaves::sellVal
+    DevBuf<unsigned char> segWords;  // (value, tag) partial sums of the long rows' segments
 };
 
 // Device copy of a gather plan (waves.h) of one sweep direction, built at
@@ -159,6 +173,11 @@ struct FuncEntry {
     std::unique_ptr<MpkPlan> mpk;
     std::unique_ptr<BlockPlan> block;  // block MPK (race_register_mpk_block)
     DevWaves waves[2];  // forward, reverse
+    DevFlow flow[2];
+    // dataflow executor, both directions: (value, tag) copy of x, x before
+    // the sweep, status word and ticket
+    DevBuf<unsigned char> flowX, flowOld;
+    DevBuf<int> flowCtl;
     DevGather gather[2];
 };
 

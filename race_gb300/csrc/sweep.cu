@@ -23,14 +23,29 @@
 //
 // Neither mode needs atomics on the transpose scatter: the coloring (leaf
 // mode) or the wave plan (wave mode) gives every written entry one writer.
+//
+// Gauss-Seidel and Kaczmarz, whose rows depend on one another, run either
+// mode's sums by dataflow (flow.cu), except where a row stands in the order
+// twice or a Kaczmarz row names a column twice; the kernels here run those,
+// and SpMV, SpMTV and SymmSpMV when a mode is asked for.
 #include <algorithm>
 #include <cstdlib>
+#include <future>
 
 #include <cuda_bf16.h>
 
 #include "engine.h"
+#include "sweep_ops.cuh"
 
 namespace race {
+
+// flow.cu
+void buildFlow(Engine &e, FuncEntry &f, int dir, const FlowOrder &fo, const std::vector<int> &rp,
+               const std::vector<int> &ptr, const std::vector<int> &rows, const std::vector<unsigned char> &huge,
+               const std::vector<int> &segFirst, const std::vector<int> &segBeg, const std::vector<int> &segEnd,
+               const std::vector<int> &waveChunk);
+void runFlow(Engine &e, FuncEntry &f, int dir, bool leaf);
+
 namespace {
 
 constexpr int kSweepThreads = 256;
@@ -73,21 +88,6 @@ __device__ bool gridBarrier(unsigned *bar, int *status) {
     }
     __syncthreads();
     return sOk != 0;
-}
-
-template <typename VT>
-__device__ __forceinline__ float toF(VT v) { return (float)v; }
-template <>
-__device__ __forceinline__ float toF<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
-
-// a*b + c in the accumulation type
-__device__ __forceinline__ double mac(double a, double b, double c) { return fma(a, b, c); }
-__device__ __forceinline__ float mac(float a, float b, float c) { return fmaf(a, b, c); }
-
-template <typename VT, typename XT>
-__device__ __forceinline__ XT ld(const VT *val, int j) {
-    if constexpr (sizeof(XT) == 8) return (XT)val[j];
-    else return toF<VT>(val[j]);
 }
 
 struct SweepArgs {
@@ -140,30 +140,6 @@ __device__ __forceinline__ void serialRow(const SweepArgs &a, int jb, int e, F &
     }
     for (; j < e; ++j) f(ld<VT, XT>(val, j), x[a.col[j]]);
 }
-
-// The four values of an entry group of the SELL copy (16-byte aligned).
-__device__ __forceinline__ void groupVals(const double *v, double out[4]) {
-    const double2 a = *(const double2 *)v, b = *(const double2 *)(v + 2);
-    out[0] = a.x;
-    out[1] = a.y;
-    out[2] = b.x;
-    out[3] = b.y;
-}
-__device__ __forceinline__ void groupVals(const float *v, float out[4]) {
-    const float4 a = *(const float4 *)v;
-    out[0] = a.x;
-    out[1] = a.y;
-    out[2] = a.z;
-    out[3] = a.w;
-}
-__device__ __forceinline__ void groupVals(const __nv_bfloat16 *v, float out[4]) {
-    const uint2 a = *(const uint2 *)v;
-    out[0] = __uint_as_float(a.x << 16);
-    out[1] = __uint_as_float(a.x & 0xffff0000u);
-    out[2] = __uint_as_float(a.y << 16);
-    out[3] = __uint_as_float(a.y & 0xffff0000u);
-}
-__device__ __forceinline__ int comp(const int4 &c, int q) { return q == 0 ? c.x : q == 1 ? c.y : q == 2 ? c.z : c.w; }
 
 // The entries of one row, as the row bodies below see them: entry k
 // (0-based, CRS order) and an in-order walk sum(x, k0, f) calling
@@ -285,9 +261,6 @@ __device__ __forceinline__ void rowWarp(const SweepArgs &a, int row, int lane);
 // grid barrier, then one warp per row combines its segments in order and
 // applies the kernel's row update (Kaczmarz: a second barrier, then the
 // scatter with the row's scale). Sums are reassociated, deterministically.
-constexpr int kHugeRow = 512;
-constexpr int kHugeSeg = 256;
-
 template <typename VT, typename XT>
 __device__ bool hugeWave(const SweepArgs &a, int r0, int r1, int gw, int nw, int lane);
 
@@ -446,13 +419,6 @@ __global__ void __launch_bounds__(kWaveThreads, 1) kWaveSweep(SweepArgs a) {
 }
 
 // ---- leaf mode: warp per leaf, lanes over a row, shuffle reductions
-
-template <typename XT>
-__device__ __forceinline__ XT warpSum(XT v) {
-#pragma unroll
-    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
 
 template <typename VT, typename XT>
 __device__ bool hugeWave(const SweepArgs &a, int r0, int r1, int gw, int nw, int lane) {
@@ -780,7 +746,8 @@ void runGather(Engine &e, FuncEntry &f, int dir) {
 // the cheaper of the two by a cost model fitted to GB300 timings (3D
 // stencils and power-law graphs): a wave costs about 12 us (barrier plus one
 // row's latency), a leaf phase about 1.3 us plus 0.67 us per row of its
-// longest leaf.
+// longest leaf. For Gauss-Seidel and Kaczmarz it picks whose sums the
+// dataflow executor computes.
 bool useWaveMode(const Engine &e, const FuncEntry &f, int dir) {
     if (e.sweepMode == SWEEP_WAVE) return f.waves[dir].numWaves > 0;
     if (e.sweepMode == SWEEP_LEAF) return false;
@@ -819,8 +786,19 @@ void buildSweepWaves(Engine &e, FuncEntry &f) {
     std::vector<int> cl(std::max(rp[n], 1));
     RACE_CUDA(cudaMemcpyAsync(cl.data(), f.ops.col, sizeof(int) * (size_t)rp[n], cudaMemcpyDeviceToHost, e.stream));
     RACE_CUDA(cudaStreamSynchronize(e.stream));
+    // both directions' orders at once: host walks over all entries
+    struct HostPlan {
+        WavePlan waves;
+        FlowOrder flow;
+    };
+    auto hostPlan = [&](int dir) {
+        return HostPlan{buildWavePlan(f.kernel, n, rp.data(), cl.data(), e.phases[dir]),
+                        buildFlowOrder(f.kernel, n, rp.data(), cl.data(), e.phases[dir])};
+    };
+    std::future<HostPlan> reverse = std::async(std::launch::async, hostPlan, 1);
     for (int dir = 0; dir < 2; ++dir) {
-        WavePlan wp = buildWavePlan(f.kernel, n, rp.data(), cl.data(), e.phases[dir]);
+        const HostPlan hp = dir == 0 ? hostPlan(0) : reverse.get();
+        const WavePlan &wp = hp.waves;
         // Rows above kHugeRow leave their wave for a wave of their own just
         // before it (rows of a wave are independent, so any split keeps the
         // order valid); their segments are listed per plan position.
@@ -905,7 +883,11 @@ void buildSweepWaves(Engine &e, FuncEntry &f) {
         w.sell = e.sweepSell;
         w.sellMidRow = mid;
         w.sellSlots = slots;
+        if (f.kernel == RACE_K_GS || f.kernel == RACE_K_KACZ)
+            buildFlow(e, f, dir, hp.flow, rp, ptr, rows, huge, segFirst, segBeg, segEnd, waveChunk);
         if (w.sell) {
+            DevFlow &fl = f.flow[dir];
+            const int *sellSrc = fl.ok && f.kernel == RACE_K_GS ? fl.mark.p : f.ops.col;
             const int C = (int)cPos.size();
             w.waveChunk.upload(waveChunk.data(), waveChunk.size(), e.stream);
             w.chunkOff.upload(cOff.empty() ? nullptr : cOff.data(), std::max(C, 1), e.stream);
@@ -920,23 +902,30 @@ void buildSweepWaves(Engine &e, FuncEntry &f) {
                 const int blocks = ceilDiv(C, 8);
                 switch (f.ops.val_type) {
                 case RACE_VAL_F64:
-                    kWaveToSell<double><<<blocks, 256, 0, e.stream>>>(f.ops.rowPtr, f.ops.col, (const double *)f.ops.val,
+                    kWaveToSell<double><<<blocks, 256, 0, e.stream>>>(f.ops.rowPtr, sellSrc, (const double *)f.ops.val,
                                                                      w.rows.p, dPos.p, dEnd.p, dLen.p, w.chunkOff.p, C,
                                                                      mid, (double *)w.sellVal.p, w.sellCol.p);
                     break;
                 case RACE_VAL_F32:
-                    kWaveToSell<float><<<blocks, 256, 0, e.stream>>>(f.ops.rowPtr, f.ops.col, (const float *)f.ops.val,
+                    kWaveToSell<float><<<blocks, 256, 0, e.stream>>>(f.ops.rowPtr, sellSrc, (const float *)f.ops.val,
                                                                     w.rows.p, dPos.p, dEnd.p, dLen.p, w.chunkOff.p, C,
                                                                     mid, (float *)w.sellVal.p, w.sellCol.p);
                     break;
                 case RACE_VAL_BF16:
                     kWaveToSell<__nv_bfloat16><<<blocks, 256, 0, e.stream>>>(
-                        f.ops.rowPtr, f.ops.col, (const __nv_bfloat16 *)f.ops.val, w.rows.p, dPos.p, dEnd.p, dLen.p,
+                        f.ops.rowPtr, sellSrc, (const __nv_bfloat16 *)f.ops.val, w.rows.p, dPos.p, dEnd.p, dLen.p,
                         w.chunkOff.p, C, mid, (__nv_bfloat16 *)w.sellVal.p, w.sellCol.p);
                     break;
                 default: throw Error(RACE_ERR_INVALID_ARG, "unknown value type");
                 }
                 RACE_CUDA(cudaGetLastError());
+                if (fl.ok && f.kernel == RACE_K_KACZ) {
+                    fl.sellMark.alloc(std::max<long long>(slots, 4));
+                    kWaveToSell<int><<<blocks, 256, 0, e.stream>>>(f.ops.rowPtr, f.ops.col, fl.mark.p, w.rows.p, dPos.p,
+                                                                   dEnd.p, dLen.p, w.chunkOff.p, C, mid, fl.sellMark.p,
+                                                                   w.sellCol.p);
+                    RACE_CUDA(cudaGetLastError());
+                }
             }
             RACE_CUDA(cudaStreamSynchronize(e.stream));  // the temporaries go out of scope
         }
@@ -952,16 +941,27 @@ bool usesGather(const Engine &e, const FuncEntry &f) {
 void runSweep(Engine &e, FuncEntry &f, bool rev) {
     const race_operands &ops = f.ops;
     const int dir = rev ? 1 : 0;
-    RACE_CUDA(cudaMemsetAsync(e.dStatus.p, 0, sizeof(int) * 4, e.stream));
     // SpMV, SpMTV and SymmSpMV have no data dependencies between rows: by
     // default (and in gather mode) they run as one gather launch, which on
     // GB300 beats the phase-by-phase executors by 9-37x on the 32^3 D2
     // SymmSpMV (0.010 ms against 0.089-0.77 ms per call)
     if (usesGather(e, f)) {
         runGather(e, f, dir);
+        e.lastStatus = nullptr;  // no device waits
         return;
     }
     const bool waveMode = useWaveMode(e, f, dir);
+    // Gauss-Seidel and Kaczmarz: by dataflow, which replaces a grid barrier
+    // per wave (or a leaf's serial walk per phase) by one L2 round trip per
+    // dependent row, with the same sums; faster at every size measured
+    // (4k rows to 100k, see flow.cu)
+    if (f.flow[dir].ok) {
+        runFlow(e, f, dir, !waveMode);
+        e.lastStatus = f.flowCtl.p;
+        return;
+    }
+    e.lastStatus = e.dStatus.p;
+    RACE_CUDA(cudaMemsetAsync(e.dStatus.p, 0, sizeof(int) * 4, e.stream));
     SweepArgs a{f.kernel, ops.rowPtr, ops.col, ops.val, ops.x, ops.b, nullptr, nullptr, nullptr, 0,
                 (unsigned *)(e.dStatus.p + 2), e.dStatus.p};
     a.midRow = midRowOf(e, f);

@@ -15,6 +15,7 @@
 #include "waves.h"
 
 #include <algorithm>
+#include <climits>
 
 namespace race {
 
@@ -51,11 +52,9 @@ struct Access {
         }
     }
 };
-}  // namespace
 
-WavePlan buildWavePlan(int kernel, int n, const int *rowPtr, const int *col, const PhaseTable &pt) {
-    WavePlan wp;
-    // rows in RACE's execution order
+// Rows in RACE's execution order.
+std::vector<int> executionOrder(int n, const PhaseTable &pt) {
     std::vector<int> order;
     order.reserve(n);
     for (size_t l = 0; l < pt.leafLo.size(); ++l) {
@@ -65,6 +64,13 @@ WavePlan buildWavePlan(int kernel, int n, const int *rowPtr, const int *col, con
         else
             for (int r = lo; r > hi; --r) order.push_back(r);
     }
+    return order;
+}
+}  // namespace
+
+WavePlan buildWavePlan(int kernel, int n, const int *rowPtr, const int *col, const PhaseTable &pt) {
+    WavePlan wp;
+    const std::vector<int> order = executionOrder(n, pt);
     // per entry: wave of the last write and of the latest read, x and b
     std::vector<int> lastW[2], lastR[2];
     for (int v = 0; v < 2; ++v) {
@@ -102,19 +108,39 @@ WavePlan buildWavePlan(int kernel, int n, const int *rowPtr, const int *col, con
     return wp;
 }
 
+FlowOrder buildFlowOrder(int kernel, int n, const int *rowPtr, const int *col, const PhaseTable &pt) {
+    FlowOrder fo;
+    if (kernel != RACE_K_GS && kernel != RACE_K_KACZ) return fo;
+    const std::vector<int> order = executionOrder(n, pt);
+    fo.order.assign(n, INT_MAX);
+    for (size_t i = 0; i < order.size(); ++i) {
+        if (fo.order[order[i]] != INT_MAX) return fo;  // a row runs twice
+        fo.order[order[i]] = (int)i;
+    }
+    for (int j = 0; j < rowPtr[n]; ++j)
+        if (col[j] < 0 || col[j] >= n) return fo;
+    if (kernel == RACE_K_KACZ) {
+        fo.mark.assign(std::max(rowPtr[n], 1), 0);
+        std::vector<int> count(n, 0), lastEntry(n, -1), lastRow(n, -1);
+        for (int r : order)
+            for (int j = rowPtr[r]; j < rowPtr[r + 1]; ++j) {
+                const int c = col[j];
+                if (lastRow[c] == r) return fo;  // the row names the column twice
+                lastRow[c] = r;
+                lastEntry[c] = j;
+                fo.mark[j] = count[c]++;
+            }
+        for (int c = 0; c < n; ++c)
+            if (lastEntry[c] >= 0) fo.mark[lastEntry[c]] |= INT_MIN;
+    }
+    fo.ok = true;
+    return fo;
+}
+
 GatherPlan buildGatherPlan(int kernel, int n, const int *rowPtr, const int *col, const PhaseTable &pt) {
     GatherPlan gp;
     if (kernel != RACE_K_SPMTV && kernel != RACE_K_SYMMSPMV) return gp;
-    // rows in RACE's execution order
-    std::vector<int> order;
-    order.reserve(n);
-    for (size_t l = 0; l < pt.leafLo.size(); ++l) {
-        const int lo = pt.leafLo[l], hi = pt.leafHi[l];
-        if (lo <= hi)
-            for (int r = lo; r < hi; ++r) order.push_back(r);
-        else
-            for (int r = lo; r > hi; --r) order.push_back(r);
-    }
+    const std::vector<int> order = executionOrder(n, pt);
     // count, then fill the updates of every b entry in execution order
     const bool symm = kernel == RACE_K_SYMMSPMV;
     std::vector<int> count(n + 1, 0);

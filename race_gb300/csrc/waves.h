@@ -18,6 +18,20 @@ struct WavePlan {
 // (host CRS) for the execution order given by a phase table.
 WavePlan buildWavePlan(int kernel, int n, const int *rowPtr, const int *col, const PhaseTable &pt);
 
+// What the dataflow executor (flow.cu) needs to know about the execution
+// order of a Gauss-Seidel or Kaczmarz function. ok: the order holds every row
+// at most once and every column is a row (and no Kaczmarz row names a column
+// twice); otherwise the sweep keeps the wave or leaf executor.
+struct FlowOrder {
+    bool ok = false;
+    std::vector<int> order;  // Gauss-Seidel: each row's place in the order (INT_MAX: not in it)
+    // Kaczmarz: per matrix entry the updates its column gets from earlier
+    // rows, with the sign bit where this row makes the last one
+    std::vector<int> mark;
+};
+
+FlowOrder buildFlowOrder(int kernel, int n, const int *rowPtr, const int *col, const PhaseTable &pt);
+
 // Gather plan of a scatter kernel (SpMTV or SymmSpMV) for one sweep
 // direction: the same updates, grouped by the entry of b they write, so
 // that every entry of b is produced by one thread in one launch. For entry
