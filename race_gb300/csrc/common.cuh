@@ -38,8 +38,11 @@ constexpr long long kSpinLimit = 1LL << 22;
 
 // Matrix-power rows longer than this are summed by a whole warp: lane l
 // takes entries l, l+32, ... as one fma chain, then an xor butterfly over
-// offsets 16, 8, 4, 2, 1 combines the 32 partial sums.
+// offsets 16, 8, 4, 2, 1 combines the 32 partial sums. FP64 rows of more than
+// kMpkHubSeg entries do so for every kMpkHubSeg of them, and lane l adds the
+// sums of segments l, l+32, ... in order before a last butterfly.
 constexpr int kMpkHubRowLen = 256;
+constexpr int kMpkHubSeg = 512;
 // Largest column window of the MPK's 16-bit column layout (14-bit offsets).
 constexpr int kMpkColWindow = 1 << 14;
 

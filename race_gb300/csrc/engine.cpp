@@ -203,8 +203,7 @@ void Engine::launch(int id, bool rev) {
         runBatch(f.block->tables, stream);
         lastStatus = f.block->tables.status.p;
     } else if (f.kernel == RACE_K_MPK) {
-        runMpk(*this, *f.mpk, f.ops, f.power);
-        lastStatus = f.mpk->status.p;
+        runMpk(*this, *f.mpk, f.ops, f.power);  // sets lastStatus
     } else {
         runSweep(*this, f, rev);  // sets lastStatus
     }

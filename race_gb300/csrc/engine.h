@@ -46,6 +46,10 @@ struct MpkPlan {
     DevBuf<int> hubRow, hubPtr; // numHubs, numHubs+1
     DevBuf<unsigned char> hubVal;  // hub entries (type valType)
     DevBuf<int> hubCol;
+    // the hub rows as work of the plain SpMV (mpk.cu HubWork)
+    int hubBig = 0, hubWork = 0;
+    DevBuf<int> hubWorkRow, hubSegFirst, hubCount;
+    DevBuf<double> hubSegPart;
     DevBuf<unsigned char> sellVal;  // sellSlots values (type valType)
     DevBuf<int> sellCol;        // sellSlots column indices (32-bit layout)
     // 16-bit layout (col16): per chunk four column window bases, per slot a

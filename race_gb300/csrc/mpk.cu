@@ -46,6 +46,7 @@
 // path issues no FP64 instructions in its inner loop.
 #include <algorithm>
 #include <numeric>
+#include <type_traits>
 
 #include <cuda_bf16.h>
 
@@ -58,6 +59,19 @@ namespace race {
 constexpr int kWarpThreads = 256;
 // Rows longer than this are summed by a whole warp from a contiguous copy.
 constexpr int kHubRowLen = kMpkHubRowLen;
+// Resident blocks per SM that the plain SpMV is compiled for (0: unbounded;
+// FP64 takes 40 registers, 6 blocks), and the warps per SM up to which every
+// warp gets at most one chunk. Measured: FP32 27-point 97x113x89, p = 8, 308 us
+// with 8 blocks and a few spilled words, 333 us with 40 registers; FP64
+// 60x61x63, p = 4, 59 us so, 64 us bounded to 6 blocks (which spills), and 66
+// us on the one-chunk kernel at two chunks a warp.
+template <typename VT>
+constexpr int kSpmvMinBlocks = sizeof(VT) == 8 ? 0 : 8;
+constexpr int kSmallWarpsPerSm = 32;
+// Hub rows of FP32/BF16 values above this length are summed by a block each
+// (two tiles). The longest row bounds a power-law matrix, so the line hardly
+// matters: 151-153 us at 512 to 8,192 for the graph below.
+constexpr int kHubBlockLen = 4096;
 
 namespace {
 
@@ -135,6 +149,18 @@ struct SellView {
     const int4 *chunkBase;
     const unsigned short *col16;
     const int *wideCol;
+};
+
+// The hub rows as work of the plain SpMV. FP64: `num` segments of kMpkHubSeg
+// entries, a warp each (hub: the row of each; first: a row's first segment;
+// count: segments finished, zero between launches; part: their sums). FP32 and
+// BF16 values: the rows by falling length (hub), the first `big` a block each,
+// the `num` others a warp each.
+struct HubWork {
+    int big, num;
+    const int *hub, *first;
+    int *count;
+    void *part;
 };
 
 // Vector loads of one entry group (four consecutive entries of a lane's
@@ -275,21 +301,49 @@ __device__ __forceinline__ void sellRow(const SellView &m, const void *col, long
     }
 }
 
-// A hub row summed by the whole warp: lane l takes entries l, l+32, ... in
-// order (one fma chain per lane, coalesced reads of the contiguous copy),
-// then a fixed butterfly combines the 32 partial sums. Deterministic, but
-// not the sequential order of the short rows: results agree with the
-// single-chain sum to rounding (relative 1e-15 scale), not bit for bit.
-template <typename VT, typename AT>
-__device__ __forceinline__ AT hubSum(const SellView &m, int h, const AT *x) {
-    const int lane = threadIdx.x & 31;
+// Sum of hub entries [beg, end) by a warp: lane l takes entries l, l+32, ...
+// in order (one fma chain per lane, coalesced reads of the contiguous copy,
+// U of them in flight), then a fixed butterfly combines the 32 partial
+// sums.
+template <typename VT, typename AT, int U>
+__device__ __forceinline__ AT hubSegment(const SellView &m, int beg, int end, const AT *x) {
     const VT *__restrict__ val = (const VT *)m.hubVal;
     AT t = AT(0);
-    for (int e = m.hubPtr[h] + lane; e < m.hubPtr[h + 1]; e += 32) {
-        if constexpr (sizeof(VT) == 8)
-            t = fma(val[e], x[m.hubCol[e]], t);
-        else
-            t = fmaf(toF<VT>(val[e]), x[m.hubCol[e]], t);
+    for (int e0 = beg + (threadIdx.x & 31); e0 < end; e0 += 32 * U) {
+        AT v[U], xv[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int e = e0 + 32 * u;
+            const bool ok = e < end;
+            if constexpr (sizeof(VT) == 8) v[u] = ok ? val[e] : AT(0);
+            else v[u] = ok ? toF<VT>(val[e]) : AT(0);
+            xv[u] = ok ? x[m.hubCol[e]] : AT(0);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (e0 + 32 * u < end) t = fma(v[u], xv[u], t);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    return t;
+}
+
+// A hub row by one warp. FP64: segments of kMpkHubSeg entries, lane l adding
+// the sums of segments l, l+32, ... in order, then the butterfly again (a
+// lane's chain of a 60k-entry row would be 1,900 FP64 fmas of 64 cycles).
+// FP32 and BF16 values: one segment. Deterministic, but not the sequential
+// order of the short rows: results agree with the single-chain sum to
+// rounding, not bit for bit. The plain SpMV shares a row among warps
+// (hubTask, hubBlock); here one warp runs it, with few loads in flight to stay
+// within the wavefront kernel's 40 registers.
+template <typename VT, typename AT>
+__device__ __forceinline__ AT hubSum(const SellView &m, int h, const AT *x) {
+    const int beg = m.hubPtr[h], end = m.hubPtr[h + 1], lane = threadIdx.x & 31;
+    if (sizeof(VT) != 8 || end - beg <= kMpkHubSeg) return hubSegment<VT, AT, 4>(m, beg, end, x);
+    AT t = AT(0);
+    for (int s = beg, g = 0; s < end; s += kMpkHubSeg, ++g) {
+        const AT p = hubSegment<VT, AT, 4>(m, s, min(end, s + kMpkHubSeg), x);
+        if (lane == (g & 31)) t += p;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
@@ -444,13 +498,215 @@ __global__ void __launch_bounds__(kWarpThreads, kMpkMinBlocks) kMpk(MpkArgs a) {
     }
 }
 
-// Plain y = A x on the SELL layout, no schedule: one warp per chunk.
-template <typename VT, bool HUBS, bool C16>
-__global__ void __launch_bounds__(kWarpThreads) kSpmvSell(SellView m, int numChunks, int n, int k, double *x,
-                                                          float *xf) {
+// Programmatic dependent launch: the next kernel of the stream may start (its
+// part before its own pdlWait) once every block of this one has; pdlWait
+// returns when the kernels before this one are complete and visible.
+__device__ __forceinline__ void pdlTrigger() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void pdlWait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// One row as sellRowAcc, the matrix read one entry group ahead of the
+// gathers of x, its first group before x may be read at all.
+template <typename VT, typename AT, bool C16>
+__device__ __forceinline__ AT sellRowAhead(const VT *__restrict__ val, long long voff, const void *col, long long coff,
+                                           int4 b, int len, const AT *x) {
+    AT t = AT(0), v[4] = {AT(0), AT(0), AT(0), AT(0)};
+    int4 c = make_int4(0, 0, 0, 0);
+    if (len > 0) {
+        groupVals<false>(val, voff, v, 0);
+        c = groupCols<C16, false>(col, coff, b, 0);
+    }
+    pdlWait();
+    for (int j = 0; j < len; j += 4) {
+        AT vn[4] = {AT(0), AT(0), AT(0), AT(0)};
+        int4 cn = make_int4(0, 0, 0, 0);
+        if (j + 4 < len) {
+            groupVals<false>(val, voff + 32LL * (j + 4), vn, 0);
+            cn = groupCols<C16, false>(col, coff + 32LL * (j + 4), b, 0);
+        }
+        if (len - j >= 4) {
+            const AT x0 = x[c.x], x1 = x[c.y], x2 = x[c.z], x3 = x[c.w];
+            t = fma(v[0], x0, t);
+            t = fma(v[1], x1, t);
+            t = fma(v[2], x2, t);
+            t = fma(v[3], x3, t);
+        } else {
+            t = fma(v[0], x[c.x], t);
+            if (len - j > 1) t = fma(v[1], x[c.y], t);
+            if (len - j > 2) t = fma(v[2], x[c.z], t);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[q] = vn[q];
+        c = cn;
+    }
+    return t;
+}
+
+// Result of row r at power k -> k+1 (FP32/BF16 also to the FP64 powers).
+__device__ __forceinline__ void putRow(double v, int r, int k, int n, double *x, float *) {
+    x[(size_t)(k + 1) * n + r] = v;
+}
+__device__ __forceinline__ void putRow(float v, int r, int k, int n, double *x, float *xf) {
+    xf[(size_t)(k + 1) * n + r] = v;
+    x[(size_t)(k + 1) * n + r] = floatToDoubleExact(v);
+}
+
+// FP64: one segment of a hub row by one warp. The warp that finishes the
+// row's last segment adds them up as hubSum does and leaves the row's counter
+// at zero for the next launch. FP32/BF16: one shorter hub row by one warp.
+template <typename VT, typename AT>
+__device__ __forceinline__ void hubTask(const SellView &m, const HubWork &hw, int i, int k, int n, const AT *xin,
+                                        double *x, float *xf) {
+    const int lane = threadIdx.x & 31;
+    if constexpr (sizeof(VT) != 8) {
+        const int h = hw.hub[hw.big + i];
+        const AT t = hubSegment<VT, AT, 8>(m, m.hubPtr[h], m.hubPtr[h + 1], xin);
+        if (lane == 0) putRow(t, m.hubRow[h], k, n, x, xf);
+    } else {
+        const int h = hw.hub[i];
+        const int first = hw.first[h], segs = hw.first[h + 1] - first;
+        const int beg = m.hubPtr[h] + (i - first) * kMpkHubSeg;
+        AT t = hubSegment<VT, AT, 8>(m, beg, min(m.hubPtr[h + 1], beg + kMpkHubSeg), xin);
+        if (segs > 1) {
+            AT *part = (AT *)hw.part;
+            int last = 0;
+            if (lane == 0) {
+                part[i] = t;
+                __threadfence();
+                last = atomicAdd(hw.count + h, 1) == segs - 1;
+            }
+            if (!__shfl_sync(0xffffffffu, last, 0)) return;
+            __threadfence();
+            t = AT(0);
+            for (int g = lane; g < segs; g += 32) t += __ldcg(part + first + g);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+            if (lane == 0) hw.count[h] = 0;
+        }
+        if (lane == 0) putRow(t, m.hubRow[h], k, n, x, xf);
+    }
+}
+
+// One long hub row (FP32/BF16) by a block: all warps gather the entries, a
+// tile of (value, x) pairs at a time, and the first runs hubSegment's 32
+// chains over the tiles, in its order. A warp alone waits for a round trip per
+// few entries of each lane; here the next tile's gathers and the columns of
+// the one after are in flight while a tile is summed.
+constexpr int kHubTile = 8 * kWarpThreads;  // entries: 16 KB of pairs
+template <typename VT>
+__device__ __forceinline__ void hubBlock(const SellView &m, int h, int k, int n, const float *xin, double *x,
+                                         float *xf) {
+    __shared__ float2 tile[kHubTile];
+    constexpr int E = kHubTile / kWarpThreads;
+    const int beg = m.hubPtr[h], end = m.hubPtr[h + 1], tid = threadIdx.x;
+    const VT *__restrict__ val = (const VT *)m.hubVal;
+    int c[E];
+    float v[E], vn[E], xv[E];
+    auto load = [&](int t0, float (&w)[E]) {  // values and columns of the tile at t0
+#pragma unroll
+        for (int i = 0; i < E; ++i) {
+            const int e = t0 + i * kWarpThreads + tid;
+            w[i] = e < end ? toF<VT>(val[e]) : 0.f;
+            c[i] = e < end ? m.hubCol[e] : -1;
+        }
+    };
+    auto gather = [&] {
+#pragma unroll
+        for (int i = 0; i < E; ++i) xv[i] = c[i] >= 0 ? xin[c[i]] : 0.f;
+    };
+    load(beg, v);
+    pdlWait();
+    gather();
+    load(beg + kHubTile, vn);
+    float t = 0.f;
+    for (int t0 = beg; t0 < end; t0 += kHubTile) {
+#pragma unroll
+        for (int i = 0; i < E; ++i) tile[i * kWarpThreads + tid] = make_float2(v[i], xv[i]);
+        __syncthreads();
+        gather();
+#pragma unroll
+        for (int i = 0; i < E; ++i) v[i] = vn[i];
+        load(t0 + 2 * kHubTile, vn);
+        if (tid < 32) {
+            const int cnt = min(kHubTile, end - t0);
+#pragma unroll 8
+            for (int i = tid; i < cnt; i += 32) t = fmaf(tile[i].x, tile[i].y, t);
+        }
+        __syncthreads();
+    }
+    if (tid < 32) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (tid == 0) putRow(t, m.hubRow[h], k, n, x, xf);
+    }
+}
+
+// Plain x_{k+1} = A x_k on the SELL layout, no schedule: one warp per hub
+// segment (they come first: the longest work) and per chunk. The next power's
+// launch overlaps this one's tail (pdlTrigger), which took 2-3 us a power:
+// 27-point 97x113x89, FP32, p = 8 (loads of 162 MB a power): 347 us before,
+// 305 us now; 7-point 32^3, FP64, p = 4 (launches): 25.3 and 14.3 us; BF16,
+// 150k-row power-law graph, p = 4: 790 us with one warp per hub row (rows of
+// up to 80k entries), 152-179 us now.
+//
+// kSpmvSell: a grid of resident warps striding the work, for matrices of
+// several chunks a warp, where loads in flight (occupancy) decide: FP32 runs
+// with 32 registers and 8 blocks an SM.
+template <typename VT, bool C16>
+__global__ void __launch_bounds__(kWarpThreads, kSpmvMinBlocks<VT>)
+    kSpmvSell(SellView m, int numChunks, int n, int k, double *x, float *xf) {
+    pdlTrigger();
+    pdlWait();
     const int nw = gridDim.x * (blockDim.x >> 5);
     for (int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < numChunks; c += nw)
-        chunkRow<VT, HUBS, C16>(m, c, k, n, x, xf, 0);
+        chunkRow<VT, false, C16>(m, c, k, n, x, xf, 0);
+}
+
+// kSpmvSellSmall: one piece of work a warp, for matrices of at most
+// kSmallWarpsPerSm chunks an SM and those with hub rows, where the chain of
+// loads of a single row decides: row tables and first entry group are read
+// before the previous power is complete, later groups one ahead of their
+// gathers, hub rows with eight gathers a lane in flight.
+template <typename VT, bool HUBS, bool C16>
+__global__ void __launch_bounds__(kWarpThreads, kSmallWarpsPerSm * 32 / kWarpThreads)
+    kSpmvSellSmall(SellView m, HubWork hw, int numChunks, int n, int k, double *x, float *xf) {
+    using AT = typename std::conditional<sizeof(VT) == 8, double, float>::type;
+    pdlTrigger();
+    const AT *xin;
+    if constexpr (sizeof(VT) == 8) xin = x + (size_t)k * n;
+    else xin = xf + (size_t)k * n;
+    int c = blockIdx.x * (kWarpThreads / 32) + (threadIdx.x >> 5);
+    if constexpr (HUBS) {
+        if constexpr (sizeof(VT) != 8) {
+            if ((int)blockIdx.x < hw.big) {
+                hubBlock<VT>(m, hw.hub[blockIdx.x], k, n, xin, x, xf);
+                return;
+            }
+            c -= hw.big * (kWarpThreads / 32);
+        }
+        if (c < hw.num) {
+            pdlWait();
+            hubTask<VT, AT>(m, hw, c, k, n, xin, x, xf);
+            return;
+        }
+        c -= hw.num;
+    }
+    if (c >= numChunks) return;
+    const int lane = threadIdx.x & 31;
+    const int r = m.chunkRow[c] + lane;
+    if (r >= m.chunkRow[c + 1]) return;
+    const int len = m.rowLen[r];
+    if (len < 0) return;  // a hub row
+    const long long off = m.chunkOff[c] + 4 * lane;
+    const VT *val = (const VT *)m.val;
+    AT t;
+    if constexpr (C16) {
+        const int4 b = m.chunkBase[c];
+        t = b.x >= 0 ? sellRowAhead<VT, AT, true>(val, off, m.col16, off, b, len, xin)
+                     : sellRowAhead<VT, AT, false>(val, off, m.wideCol, (long long)b.y + 4 * lane, b, len, xin);
+    } else {
+        t = sellRowAhead<VT, AT, false>(val, off, m.col, off, make_int4(0, 0, 0, 0), len, xin);
+    }
+    putRow(t, r, k, n, x, xf);
 }
 
 // One wavefront step of a triangular partition: one warp per (chunk,
@@ -467,6 +723,7 @@ __global__ void __launch_bounds__(kWarpThreads) kMpkStep(SellView m, const int *
 
 // x0 -> FP32 copy (rounding to nearest) for the reduced-precision path.
 __global__ void kToFloat(const double *__restrict__ x, float *__restrict__ xf, int n) {
+    pdlTrigger();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) xf[i] = (float)x[i];
 }
@@ -733,6 +990,28 @@ std::unique_ptr<MpkPlan> buildMpkPlan(Engine &e, const race_operands &ops, int p
     plan->hubPtr.upload(hubPtrH.data(), hubPtrH.size(), s);
     plan->hubVal.alloc(std::max<long long>(hubPtrH.back(), 1) * valBytes(ops.val_type));
     plan->hubCol.alloc(std::max<long long>(hubPtrH.back(), 1));
+    if (H) {
+        // hub rows as work of the plain SpMV (HubWork)
+        std::vector<int> work, segFirst{0};
+        auto hubLen = [&](int h) { return hubPtrH[h + 1] - hubPtrH[h]; };
+        for (int h = 0; h < H; ++h) {
+            const int segs = ceilDiv(hubLen(h), kMpkHubSeg);
+            if (ops.val_type == RACE_VAL_F64) work.insert(work.end(), segs, h);
+            else work.push_back(h);
+            segFirst.push_back(segFirst.back() + segs);
+        }
+        if (ops.val_type != RACE_VAL_F64) {
+            std::stable_sort(work.begin(), work.end(), [&](int a, int b) { return hubLen(a) > hubLen(b); });
+            while (plan->hubBig < H && hubLen(work[plan->hubBig]) > kHubBlockLen) ++plan->hubBig;
+        }
+        plan->hubWork = (int)work.size() - plan->hubBig;
+        plan->hubWorkRow.upload(work.data(), work.size(), s);
+        plan->hubSegFirst.upload(segFirst.data(), segFirst.size(), s);
+        plan->hubSegPart.alloc(segFirst.back());
+        plan->hubCount.alloc(H);
+        RACE_CUDA(cudaMemsetAsync(plan->hubCount.p, 0, sizeof(int) * H, s));
+        RACE_CUDA(cudaStreamSynchronize(s));  // work and segFirst go out of scope
+    }
     plan->numChunks = C;
     plan->power = power;
     plan->valType = ops.val_type;
@@ -963,20 +1242,35 @@ void launchMpkSteps(const MpkPlan &p, int n, double *x, cudaStream_t s) {
 }
 
 template <typename VT, bool HUBS, bool C16>
-void launchSpmvSellK(const SellView &v, int numChunks, int n, int k, double *x, float *xf, cudaStream_t s) {
-    static int blocks = residentBlocks(kSpmvSell<VT, HUBS, C16>, kWarpThreads);
-    kSpmvSell<VT, HUBS, C16><<<blocks, kWarpThreads, 0, s>>>(v, numChunks, n, k, x, xf);
+void launchSpmvSellK(const MpkPlan &p, int n, int k, double *x, cudaStream_t s) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.blockDim = dim3(kWarpThreads);
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    const int blocks = std::max(1, ceilDiv((long long)p.hubWork + p.numChunks, kWarpThreads / 32));
+    if (HUBS || p.numChunks <= kSmallWarpsPerSm * devSms()) {
+        const HubWork hw{p.hubBig, p.hubWork, p.hubWorkRow.p, p.hubSegFirst.p, p.hubCount.p, p.hubSegPart.p};
+        cfg.gridDim = dim3(p.hubBig + blocks);
+        RACE_CUDA(cudaLaunchKernelEx(&cfg, kSpmvSellSmall<VT, HUBS, C16>, viewOf(p), hw, p.numChunks, n, k, x, p.xf.p));
+        return;
+    }
+    static const int resident = residentBlocks(kSpmvSell<VT, C16>, kWarpThreads);
+    cfg.gridDim = dim3(std::min(resident, blocks));
+    RACE_CUDA(cudaLaunchKernelEx(&cfg, kSpmvSell<VT, C16>, viewOf(p), p.numChunks, n, k, x, p.xf.p));
 }
 
 template <typename VT>
 void launchSpmvSell(const MpkPlan &p, int n, int k, double *x, cudaStream_t s) {
-    const SellView v = viewOf(p);
     if (p.numHubs > 0) {
-        if (p.col16) launchSpmvSellK<VT, true, true>(v, p.numChunks, n, k, x, p.xf.p, s);
-        else launchSpmvSellK<VT, true, false>(v, p.numChunks, n, k, x, p.xf.p, s);
+        if (p.col16) launchSpmvSellK<VT, true, true>(p, n, k, x, s);
+        else launchSpmvSellK<VT, true, false>(p, n, k, x, s);
     } else {
-        if (p.col16) launchSpmvSellK<VT, false, true>(v, p.numChunks, n, k, x, p.xf.p, s);
-        else launchSpmvSellK<VT, false, false>(v, p.numChunks, n, k, x, p.xf.p, s);
+        if (p.col16) launchSpmvSellK<VT, false, true>(p, n, k, x, s);
+        else launchSpmvSellK<VT, false, false>(p, n, k, x, s);
     }
 }
 }  // namespace
@@ -984,6 +1278,7 @@ void launchSpmvSell(const MpkPlan &p, int n, int k, double *x, cudaStream_t s) {
 namespace {
 // The persistent wavefront kernel over all powers.
 void runWavefront(MpkPlan &plan, const race_operands &ops, cudaStream_t s) {
+    RACE_CUDA(cudaMemsetAsync(plan.status.p, 0, sizeof(int), s));
     RACE_CUDA(cudaMemsetAsync(plan.done.p, 0, sizeof(int) * (size_t)plan.numBlocks * plan.power, s));
     RACE_CUDA(cudaMemsetAsync(plan.ticket.p, 0, sizeof(int) * 2, s));
     MpkArgs a{viewOf(plan),
@@ -1024,9 +1319,11 @@ void runSweeps(MpkPlan &plan, const race_operands &ops, cudaStream_t s) {
 }
 
 // RACE_MPK_AUTO's choice: each schedule timed on its second run (the first
-// warms the code and the caches), the faster kept. Both compute the same
-// powers, so the call's result is complete either way; the wavefront's
-// status word is cleared afterwards, as the sweeps would leave it.
+// warms the code and the caches), the faster kept; a first run more than
+// twice as slow as the other's settles it (a small matrix's or a hub-row
+// matrix's wavefront is 4 to 25 times slower). Both compute the same powers,
+// so the call's result is complete either way; the wavefront's status word is
+// cleared afterwards, as the sweeps would leave it.
 int chooseSchedule(MpkPlan &plan, const race_operands &ops, cudaStream_t s) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     RACE_CUDA(cudaStreamIsCapturing(s, &cs));
@@ -1035,7 +1332,8 @@ int chooseSchedule(MpkPlan &plan, const race_operands &ops, cudaStream_t s) {
     RACE_CUDA(cudaEventCreate(&ev[0]));
     RACE_CUDA(cudaEventCreate(&ev[1]));
     float ms[2] = {0.f, 0.f};
-    for (int rep = 0; rep < 2; ++rep)
+    for (int rep = 0; rep < 2; ++rep) {
+        if (rep == 1 && (ms[0] > 2 * ms[1] || ms[1] > 2 * ms[0])) break;
         for (int sc = 0; sc < 2; ++sc) {
             RACE_CUDA(cudaEventRecord(ev[0], s));
             if (sc == 0) runWavefront(plan, ops, s);
@@ -1044,6 +1342,7 @@ int chooseSchedule(MpkPlan &plan, const race_operands &ops, cudaStream_t s) {
             RACE_CUDA(cudaEventSynchronize(ev[1]));
             RACE_CUDA(cudaEventElapsedTime(&ms[sc], ev[0], ev[1]));
         }
+    }
     cudaEventDestroy(ev[0]);
     cudaEventDestroy(ev[1]);
     int st = DEV_OK;
@@ -1058,7 +1357,7 @@ int chooseSchedule(MpkPlan &plan, const race_operands &ops, cudaStream_t s) {
 void runMpk(Engine &e, MpkPlan &plan, const race_operands &ops, int power) {
     if (power != plan.power) throw Error(RACE_ERR_INVALID_ARG, "power differs from the planned power");
     cudaStream_t s = e.stream;
-    RACE_CUDA(cudaMemsetAsync(plan.status.p, 0, sizeof(int), s));
+    e.lastStatus = nullptr;  // the plain launches wait for nothing
     if (plan.valType != RACE_VAL_F64) kToFloat<<<ceilDiv(ops.n, 256), 256, 0, s>>>((const double *)ops.x, plan.xf.p, ops.n);
     if (plan.stepped) {
         switch (plan.valType) {
@@ -1071,13 +1370,20 @@ void runMpk(Engine &e, MpkPlan &plan, const race_operands &ops, int power) {
         return;
     }
     const int sched = plan.schedule != RACE_MPK_AUTO ? plan.schedule : plan.chosen;
-    if (sched == RACE_MPK_WAVEFRONT) runWavefront(plan, ops, s);
-    else if (sched == RACE_MPK_SWEEPS) runSweeps(plan, ops, s);
-    else {
+    if (sched == RACE_MPK_WAVEFRONT) {
+        e.lastStatus = plan.status.p;
+        runWavefront(plan, ops, s);
+    } else if (sched == RACE_MPK_SWEEPS) {
+        runSweeps(plan, ops, s);
+    } else {
         const int c = chooseSchedule(plan, ops, s);
         if (plan.chosen == 0) {  // not timed (stream capture): run the default
-            if (c == RACE_MPK_WAVEFRONT) runWavefront(plan, ops, s);
-            else runSweeps(plan, ops, s);
+            if (c == RACE_MPK_WAVEFRONT) {
+                e.lastStatus = plan.status.p;
+                runWavefront(plan, ops, s);
+            } else {
+                runSweeps(plan, ops, s);
+            }
         }
     }
 }

@@ -191,14 +191,23 @@ __global__ void __launch_bounds__(kNaThreads) kMpkNoAlloc(NaArgs a) {
             a.x[(size_t)(k + 1) * a.n + r] = t;
         }
         // rows longer than kMpkHubRowLen: the whole warp, in the registered
-        // path's order (lane l: entries l, l+32, ...; then the xor butterfly)
+        // path's order (per kMpkHubSeg entries lane l: entries l, l+32, ...;
+        // then the xor butterfly; lane l: segments l, l+32, ...; butterfly)
         unsigned hubs = __ballot_sync(0xffffffffu, live && e - s > kMpkHubRowLen);
         while (hubs) {
             const int h = __ffs(hubs) - 1;
             hubs &= hubs - 1;
             const int hs = __shfl_sync(0xffffffffu, s, h), he = __shfl_sync(0xffffffffu, e, h);
             double t = 0.0;
-            for (int j = hs + lane; j < he; j += 32) t = fma(a.val[j], xin[a.col[j]], t);
+            for (int b = hs, g = 0; b < he; b += kMpkHubSeg, ++g) {
+                const int end = min(he, b + kMpkHubSeg);
+                double p = 0.0;
+                for (int j = b + lane; j < end; j += 32) p = fma(a.val[j], xin[a.col[j]], p);
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) p += __shfl_xor_sync(0xffffffffu, p, o);
+                if (lane == (g & 31)) t += p;
+            }
+            // one segment: lane 0 holds its sum, the others zeros
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
             if (lane == 0) a.x[(size_t)(k + 1) * a.n + r0 + h] = t;
