@@ -163,11 +163,16 @@ struct DevFlow {
     DevBuf<unsigned char> segWords;  // (value, tag) partial sums of the long rows' segments
 };
 
-// Device copy of a gather plan (waves.h) of one sweep direction, built at
-// the first gather-mode call.
+// Device copy of a gather plan (waves.h) of one sweep direction and its
+// layout per 32 entries of b (gather.cu), built at the first gather-mode call
+// (SpMV: at registration, in the forward direction's place).
 struct DevGather {
     bool built = false;
-    DevBuf<int> ptr, entry, row;
+    int numLong = 0;
+    DevBuf<int> mem;  // holds all of the tables below
+    long long *listOff = nullptr;
+    int *len = nullptr, *longY = nullptr, *ptr = nullptr, *entry = nullptr, *row = nullptr, *listPos = nullptr,
+        *listSrc = nullptr;
 };
 
 struct FuncEntry {

@@ -45,6 +45,9 @@ void buildFlow(Engine &e, FuncEntry &f, int dir, const FlowOrder &fo, const std:
                const std::vector<int> &segFirst, const std::vector<int> &segBeg, const std::vector<int> &segEnd,
                const std::vector<int> &waveChunk);
 void runFlow(Engine &e, FuncEntry &f, int dir, bool leaf);
+// gather.cu
+void buildGather(Engine &e, FuncEntry &f, int dir, const std::vector<int> &rp, const std::vector<int> &cl);
+void runGather(Engine &e, FuncEntry &f, int dir);
 
 namespace {
 
@@ -661,85 +664,6 @@ void launch(bool waveMode, SweepArgs &a, int maxWork, cudaStream_t s) {
     }
 }
 
-// Gather execution (RACE_SWEEP_GATHER): one thread per entry of b, which
-// replays the updates RACE's sequential walk makes to it, in that walk's
-// order (GatherPlan, waves.h), with the kernel bodies' own operations, so
-// the results equal the wave executor's bit for bit; no phases, no grid
-// barriers. SpMV needs no plan: its rows are independent.
-template <typename VT, typename XT>
-__global__ void kGather(int kernel, int n, const int *__restrict__ ptr, const int *__restrict__ entry,
-                        const int *__restrict__ src, const int *__restrict__ rowPtr, const int *__restrict__ col,
-                        const void *val_, const XT *__restrict__ x, XT *__restrict__ b) {
-    const VT *val = (const VT *)val_;
-    for (int y = blockIdx.x * blockDim.x + threadIdx.x; y < n; y += gridDim.x * blockDim.x) {
-        if (kernel == RACE_K_SPMV) {  // kernels.cpp:5-15
-            XT t = XT(0);
-            for (int j = rowPtr[y]; j < rowPtr[y + 1]; ++j) t = mac(ld<VT, XT>(val, j), x[col[j]], t);
-            b[y] = t;
-            continue;
-        }
-        XT acc = b[y];
-        for (int k = ptr[y]; k < ptr[y + 1]; ++k) {
-            const int e = entry[k];
-            if (e >= 0) {  // b[y] += a x[src] of another row (SpMTV :107-115, SymmSpMV :403-417)
-                acc = mac(ld<VT, XT>(val, e), x[src[k]], acc);
-            } else {  // row y's own SymmSpMV update: diagonal, then its off-diagonal dot product
-                const int s = rowPtr[y], end = rowPtr[y + 1];
-                if (end == s) continue;  // no diagonal entry to read
-                acc = mac(ld<VT, XT>(val, s), x[y], acc);
-                XT t = XT(0);
-                for (int j = s + 1; j < end; ++j) t = mac(ld<VT, XT>(val, j), x[col[j]], t);
-                acc += t;
-            }
-        }
-        b[y] = acc;
-    }
-}
-
-template <typename VT, typename XT>
-void launchGather(const FuncEntry &f, const DevGather &g, cudaStream_t s) {
-    const race_operands &o = f.ops;
-    const int n = o.n;
-    if (n == 0) return;
-    const int blocks = std::min(ceilDiv(n, 256), 152 * 16);
-    kGather<VT, XT><<<blocks, 256, 0, s>>>(f.kernel, n, g.ptr.p, g.entry.p, g.row.p, o.rowPtr, o.col, o.val,
-                                            (const XT *)o.x, (XT *)o.b);
-    RACE_CUDA(cudaGetLastError());
-}
-
-void runGather(Engine &e, FuncEntry &f, int dir) {
-    const race_operands &ops = f.ops;
-    DevGather &g = f.gather[dir];
-    if (!g.built && f.kernel != RACE_K_SPMV) {
-        const int n = ops.n;
-        std::vector<int> rp(n + 1);
-        RACE_CUDA(cudaMemcpyAsync(rp.data(), ops.rowPtr, sizeof(int) * (n + 1), cudaMemcpyDeviceToHost, e.stream));
-        RACE_CUDA(cudaStreamSynchronize(e.stream));
-        std::vector<int> cl(std::max(rp[n], 1));
-        RACE_CUDA(cudaMemcpyAsync(cl.data(), ops.col, sizeof(int) * (size_t)rp[n], cudaMemcpyDeviceToHost, e.stream));
-        RACE_CUDA(cudaStreamSynchronize(e.stream));
-        const GatherPlan gp = buildGatherPlan(f.kernel, n, rp.data(), cl.data(), e.phases[dir]);
-        g.ptr.upload(gp.ptr.data(), gp.ptr.size(), e.stream);
-        g.entry.upload(gp.entry.empty() ? nullptr : gp.entry.data(), std::max<size_t>(gp.entry.size(), 1), e.stream);
-        g.row.upload(gp.row.empty() ? nullptr : gp.row.data(), std::max<size_t>(gp.row.size(), 1), e.stream);
-        RACE_CUDA(cudaStreamSynchronize(e.stream));
-        g.built = true;
-    }
-    if (ops.vec_type == RACE_VAL_F64) {
-        if (ops.val_type != RACE_VAL_F64) throw Error(RACE_ERR_INVALID_ARG, "FP64 vectors need FP64 values");
-        launchGather<double, double>(f, g, e.stream);
-    } else if (ops.vec_type == RACE_VAL_F32) {
-        if (ops.val_type == RACE_VAL_F32)
-            launchGather<float, float>(f, g, e.stream);
-        else if (ops.val_type == RACE_VAL_BF16)
-            launchGather<__nv_bfloat16, float>(f, g, e.stream);
-        else
-            throw Error(RACE_ERR_INVALID_ARG, "FP32 vectors need FP32 or BF16 values");
-    } else {
-        throw Error(RACE_ERR_INVALID_ARG, "unknown vector type");
-    }
-}
-
 }  // namespace
 
 // Execution mode of one sweep direction: the engine's setting, or (auto)
@@ -786,6 +710,7 @@ void buildSweepWaves(Engine &e, FuncEntry &f) {
     std::vector<int> cl(std::max(rp[n], 1));
     RACE_CUDA(cudaMemcpyAsync(cl.data(), f.ops.col, sizeof(int) * (size_t)rp[n], cudaMemcpyDeviceToHost, e.stream));
     RACE_CUDA(cudaStreamSynchronize(e.stream));
+    if (f.kernel == RACE_K_SPMV) buildGather(e, f, 0, rp, cl);
     // both directions' orders at once: host walks over all entries
     struct HostPlan {
         WavePlan waves;
