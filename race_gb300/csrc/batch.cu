@@ -17,15 +17,23 @@
 // to p sequential fma SpMVs per right-hand side. The lanes of one row read
 // the same value and column (a broadcast) and R consecutive x entries.
 //
-// Schedule: chunks of <= 32 rows inside level groups; a work item is
-// (power, chunk); items of one member follow the stride-2 wavefront of the
-// single-vector kernel and members follow each other. Persistent warps take
-// items from a global ticket; an item waits (bounded) for the chunks of the
-// previous power its columns fall in. Dependencies stay inside a member and
-// point to earlier tickets, so the launch cannot deadlock; the next member's
-// items fill the warps that the tail of the previous member's wavefront
-// leaves idle. A batch is one memset of the completion flags plus one
-// kernel, and can be captured once in a CUDA graph and replayed.
+// Schedule: chunks of a few dozen rows inside level groups (blockChunkRows);
+// a work item is (power, chunk). The chunks of all members are numbered
+// through, and the items are listed by c + k lag (k the power, c the chunk):
+// power k of a chunk follows its power k-1 by `lag` chunks, as many as the
+// GPU has in flight and more than any chunk's inputs lie ahead of it, so that
+// inputs are complete when an item is taken, and the list holds every item
+// after its inputs. Persistent warps take items from a global ticket; an item
+// waits (bounded) for the chunks of the previous power its columns fall in.
+// Dependencies stay inside a member and point to earlier tickets, so the
+// launch cannot deadlock. A batch is one memset of the completion flags plus
+// one kernel, and can be captured once in a CUDA graph and replayed.
+//
+// Measured on GB300, p = 4 (before: items of 32 rows, one member's powers
+// right behind one another, so that most warps waited): 24 matrices of 100^2
+// to 500^2, 8 FP32 right-hand sides, 587 and 254 us; 16 of 100^2 to 700^2, 16
+// FP64 ones, 2,015 and 1,832 us, 94 % of the FP64 pipe's time (1.08 G fma at 2
+// a cycle and SM); one of about 120^2, 16 FP32 ones, 62 and 51 us.
 #include <algorithm>
 
 #include <cuda_bf16.h>
@@ -46,6 +54,32 @@ __device__ __forceinline__ int ldAcquireB(const int *p) {
     asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
+__device__ __forceinline__ int ldRelaxedB(const int *p) {
+    int v;
+    asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
+// Rows that a warp takes at once, and the most rows of an item: 4 KB of one
+// power's right-hand sides, 32 to 128 rows. Each item costs a ticket (one
+// address for the whole GPU), its table entry, the poll of its inputs and a
+// release; 32 rows of 8 FP32 right-hand sides are less work than that.
+int blockPassRows(int nrhs, int vecType) {
+    return 32 / std::max(1, nrhs * (vecType == RACE_VAL_F64 ? 8 : 4) / 16);
+}
+int blockMaxRows(int nrhs, int vecType) {
+    const int rows = 4096 / (nrhs * (vecType == RACE_VAL_F64 ? 8 : 4));
+    return std::min(128, std::max(32, rows & ~31));
+}
+// Rows of an item where `rows` rows in all are shared by `warps` warps: whole
+// passes, so that every warp has some before any takes more than one pass.
+// Measured with the most rows throughout instead: 5 matrices of 100^2 to
+// 200^2 with 8 FP64 right-hand sides 154 us (115 us with 32 rows).
+int blockItemRows(long long rows, int warps, int nrhs, int vecType) {
+    const int pass = blockPassRows(nrhs, vecType);
+    const long long share = rows / std::max(warps, 1) / pass * pass;
+    return (int)std::min<long long>(blockMaxRows(nrhs, vecType), std::max<long long>(pass, share));
+}
 
 __device__ __forceinline__ double mulAdd(double v, double x, double acc) { return fma(v, x, acc); }
 __device__ __forceinline__ float mulAdd(float v, float x, float acc) { return fmaf(v, x, acc); }
@@ -55,10 +89,10 @@ __device__ __forceinline__ float mulAdd(__nv_bfloat16 v, float x, float acc) {
 
 struct BlockArgs {
     const BlockMember *members;
-    const int *chunkMember, *chunkRow, *chunkEnd;
-    const int *depRange;
-    const int *itemChunk;
-    const unsigned char *itemPow;
+    // three per item: {first row, end row, member, power}, then three chunk
+    // ranges [lo, hi] read at the previous power and the item's own chunk:
+    // {lo0, hi0, lo1, hi1}, {lo2, hi2, chunk, 0}
+    const int4 *item;
     int numItems, numChunks;
     int *done, *ticket, *status;
 };
@@ -105,7 +139,9 @@ __device__ __forceinline__ void blockRows(const BlockMember &m, int r0, int r1, 
             Vec acc;
 #pragma unroll
             for (int t = 0; t < V; ++t) acc.v[t] = XT(0);
-#pragma unroll 4
+            // two entries at a time: four keep 13 % fewer warps' x rows in the L1
+            // (254 and 281 us for the FP32 batch above)
+#pragma unroll 2
             for (int e = e0; e < e1; ++e) {
                 const VT a = val[e];
                 const Vec xv = *reinterpret_cast<const Vec *>(xin + (size_t)col[e] * R);
@@ -117,6 +153,8 @@ __device__ __forceinline__ void blockRows(const BlockMember &m, int r0, int r1, 
     }
 }
 
+// Relaxed polls and one acquire fence after the successful one (an acquire
+// load per flag empties the L1 each time).
 template <typename VT, typename XT, int R>
 __global__ void __launch_bounds__(kBlockThreads) kMpkBlock(BlockArgs a) {
     const int lane = threadIdx.x & 31;
@@ -125,18 +163,17 @@ __global__ void __launch_bounds__(kBlockThreads) kMpkBlock(BlockArgs a) {
         if (lane == 0) it = atomicAdd(a.ticket, 1);
         it = __shfl_sync(0xffffffffu, it, 0);
         if (it >= a.numItems) return;
-        const int t = a.itemChunk[it];
-        const int k = a.itemPow[it];
+        const int4 h = a.item[3 * (size_t)it], d0 = a.item[3 * (size_t)it + 1], d1 = a.item[3 * (size_t)it + 2];
+        const int k = h.w;
+        const BlockMember m = a.members[h.z];
         if (k > 0) {
-            const int *rg = a.depRange + 6 * t;
             const int *done = a.done + (size_t)(k - 1) * a.numChunks;
             long long spins = 0;
             for (;;) {
                 bool ok = true;
-#pragma unroll
-                for (int d = 0; d < 3; ++d)
-                    for (int i = rg[2 * d] + lane; i <= rg[2 * d + 1]; i += 32)
-                        if (ldAcquireB(done + i) == 0) ok = false;
+                for (int i = d0.x + lane; i <= d0.y; i += 32) ok &= ldRelaxedB(done + i) != 0;
+                for (int i = d0.z + lane; i <= d0.w; i += 32) ok &= ldRelaxedB(done + i) != 0;
+                for (int i = d1.x + lane; i <= d1.y; i += 32) ok &= ldRelaxedB(done + i) != 0;
                 if (__all_sync(0xffffffffu, ok)) break;
                 if (++spins > kSpinLimit || ldAcquireB(a.status) != DEV_OK) {
                     if (lane == 0) atomicCAS(a.status, DEV_OK, DEV_WAIT_TIMEOUT);
@@ -144,12 +181,12 @@ __global__ void __launch_bounds__(kBlockThreads) kMpkBlock(BlockArgs a) {
                 }
                 __nanosleep(32);
             }
+            asm volatile("fence.acq_rel.gpu;" ::: "memory");
         }
-        const BlockMember m = a.members[a.chunkMember[t]];
-        blockRows<VT, XT, R>(m, a.chunkRow[t], a.chunkEnd[t], k);
+        for (int r = h.x; r < h.y; r += 32) blockRows<VT, XT, R>(m, r, min(h.y, r + 32), k);
         __syncwarp();
         if (lane == 0)
-            asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(a.done + (size_t)k * a.numChunks + t), "r"(1)
+            asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(a.done + (size_t)k * a.numChunks + d1.z), "r"(1)
                          : "memory");
     }
 }
@@ -174,9 +211,13 @@ int residentBlocksOf(K kernel) {
 }
 
 template <typename VT, typename XT, int R>
-void launchBlock(const BlockArgs &a, cudaStream_t s) {
+int blockResident() {
     static const int blocks = residentBlocksOf(kMpkBlock<VT, XT, R>);
-    kMpkBlock<VT, XT, R><<<blocks, kBlockThreads, 0, s>>>(a);
+    return blocks;
+}
+template <typename VT, typename XT, int R>
+void launchBlock(const BlockArgs &a, cudaStream_t s) {
+    kMpkBlock<VT, XT, R><<<blockResident<VT, XT, R>(), kBlockThreads, 0, s>>>(a);
 }
 
 template <typename VT, typename XT, int R>
@@ -213,9 +254,20 @@ struct LaunchBlockFn {
     static void run(const BlockArgs &a, cudaStream_t s) { launchBlock<VT, XT, R>(a, s); }
 };
 template <typename VT, typename XT, int R>
+struct WarpsInFlightFn {
+    static void run(int &warps) { warps = blockResident<VT, XT, R>() * (kBlockThreads / 32); }
+};
+template <typename VT, typename XT, int R>
 struct LaunchSpmvFn {
     static void run(const BlockMember &m, int k, cudaStream_t s) { launchSpmv<VT, XT, R>(m, k, s); }
 };
+
+// Warps of a batch launch: its items in flight.
+int blockWarpsInFlight(int valType, int vecType, int nrhs) {
+    int warps = 0;
+    dispatch<WarpsInFlightFn>(valType, vecType, nrhs, warps);
+    return warps;
+}
 
 }  // namespace
 
@@ -235,41 +287,68 @@ void buildBatchTables(BatchTables &t, const std::vector<const BlockPlan *> &plan
     t.nrhs = p0.nrhs;
     t.maxPower = 0;
     std::vector<BlockMember> mem;
-    std::vector<int> cMember, cRow, cEnd, range, iChunk;
-    std::vector<unsigned char> iPow;
-    int base = 0;
+    long long rows = 0;
+    for (const BlockPlan *p : plans) {
+        if (p->valType != t.valType || p->vecType != t.vecType || p->nrhs != t.nrhs)
+            throw Error(RACE_ERR_INCOMPATIBILITY, "batch members differ in value type, vector type or nrhs");
+        t.maxPower = std::max(t.maxPower, p->power);
+        mem.push_back(BlockMember{p->ops.rowPtr, p->ops.col, p->ops.val, p->ops.x, p->n, p->power});
+        rows += p->n;
+    }
+    // A batch's chunks: consecutive chunks of a member's plan and level group
+    // put together up to the rows that the whole batch leaves each warp.
+    const int warps = blockWarpsInFlight(t.valType, t.vecType, t.nrhs);
+    const int limit = blockItemRows(rows, warps, t.nrhs, t.vecType);
+    struct Chunk {
+        int row0, row1, member;
+        int lo[3], hi[3];  // chunks read (empty: [0, -1])
+    };
+    std::vector<Chunk> chunks;
+    int reach = 0;
     for (size_t m = 0; m < plans.size(); ++m) {
         const BlockPlan &p = *plans[m];
-        if (p.valType != t.valType || p.vecType != t.vecType || p.nrhs != t.nrhs)
-            throw Error(RACE_ERR_INCOMPATIBILITY, "batch members differ in value type, vector type or nrhs");
-        t.maxPower = std::max(t.maxPower, p.power);
-        mem.push_back(BlockMember{p.ops.rowPtr, p.ops.col, p.ops.val, p.ops.x, p.n, p.power});
+        const size_t before = chunks.size();
+        std::vector<int> of(p.numChunks);  // chunk of the batch
         for (int c = 0; c < p.numChunks; ++c) {
-            cMember.push_back((int)m);
-            cRow.push_back(p.chunkRow[c]);
-            cEnd.push_back(p.chunkRow[c + 1]);
+            const bool join = chunks.size() > before && c > 0 && p.chunkGroup[c] == p.chunkGroup[c - 1] &&
+                              p.chunkRow[c + 1] - chunks.back().row0 <= limit;
+            if (join) chunks.back().row1 = p.chunkRow[c + 1];
+            else chunks.push_back(Chunk{p.chunkRow[c], p.chunkRow[c + 1], (int)m, {0, 0, 0}, {-1, -1, -1}});
+            of[c] = (int)chunks.size() - 1;
+        }
+        for (int c = 0; c < p.numChunks; ++c)
             for (int d = 0; d < 3; ++d) {
-                const int lo = p.depRange[6 * c + 2 * d], hi = p.depRange[6 * c + 2 * d + 1];
-                range.push_back(hi < lo ? 0 : lo + base);  // empty stays empty: [0,-1]
-                range.push_back(hi < lo ? -1 : hi + base);
+                const int lo = p.depRange[6 * (size_t)c + 2 * d], hi = p.depRange[6 * (size_t)c + 2 * d + 1];
+                if (hi < lo) continue;
+                Chunk &u = chunks[of[c]];
+                u.lo[d] = u.hi[d] < 0 ? of[lo] : std::min(u.lo[d], of[lo]);
+                u.hi[d] = std::max(u.hi[d], of[hi]);
+                reach = std::max(reach, of[hi] - of[c]);
             }
-        }
-        for (size_t i = 0; i < p.itemChunk.size(); ++i) {
-            iChunk.push_back(p.itemChunk[i] + base);
-            iPow.push_back(p.itemPow[i]);
-        }
-        base += p.numChunks;
     }
+    const int base = (int)chunks.size();
     t.numMembers = (int)plans.size();
     t.numChunks = base;
-    t.numItems = (int)iChunk.size();
+    // items by c + k lag (a lag of all chunks already is power by power);
+    // twice the warps in flight: 281 us instead of 287 us at once that many
+    const int lag = std::max(1, std::min(base, std::max(reach + 1, 2 * warps)));
+    std::vector<int4> item;
+    size_t total = 0;
+    for (const Chunk &u : chunks) total += plans[u.member]->power;
+    item.reserve(3 * std::max<size_t>(total, 1));
+    for (long long at = 0; at < base + (long long)(t.maxPower - 1) * lag; ++at)
+        for (int k = (int)std::min<long long>(at / lag, t.maxPower - 1); k >= 0; --k) {
+            const long long c = at - (long long)k * lag;
+            if (c >= base) break;
+            const Chunk &u = chunks[c];
+            if (k >= plans[u.member]->power) continue;
+            item.push_back(make_int4(u.row0, u.row1, u.member, k));
+            item.push_back(make_int4(u.lo[0], u.hi[0], u.lo[1], u.hi[1]));
+            item.push_back(make_int4(u.lo[2], u.hi[2], (int)c, 0));
+        }
+    t.numItems = (int)(item.size() / 3);
     t.members.upload(mem.data(), mem.size(), s);
-    t.chunkMember.upload(cMember.data(), std::max<size_t>(cMember.size(), 1), s);
-    t.chunkRow.upload(cRow.data(), std::max<size_t>(cRow.size(), 1), s);
-    t.chunkEnd.upload(cEnd.data(), std::max<size_t>(cEnd.size(), 1), s);
-    t.depRange.upload(range.data(), std::max<size_t>(range.size(), 1), s);
-    t.itemChunk.upload(iChunk.data(), std::max<size_t>(iChunk.size(), 1), s);
-    t.itemPow.upload(iPow.data(), std::max<size_t>(iPow.size(), 1), s);
+    t.item.upload(item.empty() ? nullptr : item.data(), std::max<size_t>(item.size(), 1), s);
     t.done.alloc(std::max<size_t>((size_t)t.maxPower * t.numChunks, 1));
     t.ticket.alloc(1);
     t.status.alloc(1);
@@ -295,30 +374,19 @@ std::unique_ptr<BlockPlan> buildBlockPlan(Engine &e, const race_operands &ops, i
     const int G = (int)gp.size() - 1;
     std::vector<int> chunkGroup;
     plan->chunkRow.assign(1, 0);
+    const int rows =
+        blockItemRows(ops.n, blockWarpsInFlight(ops.val_type, ops.vec_type, nrhs), nrhs, ops.vec_type);
     for (int g = 0; g < G; ++g)
-        for (int r = gp[g]; r < gp[g + 1]; r += 32) {
-            plan->chunkRow.push_back(std::min(gp[g + 1], r + 32));
+        for (int r = gp[g]; r < gp[g + 1]; r += rows) {
+            plan->chunkRow.push_back(std::min(gp[g + 1], r + rows));
             chunkGroup.push_back(g);
         }
     const int C = (int)chunkGroup.size();
     plan->numChunks = C;
+    plan->chunkGroup = chunkGroup;
     if (!chunkDependencyRanges(ops.rowPtr, ops.col, plan->chunkRow, chunkGroup, plan->depRange, e.stream))
         throw Error(RACE_ERR_INVALID_ARG,
                     "MPK operand is not in the engine's level order (permute it with getPerm/getInvPerm)");
-    // stride-2 wavefront over (group, power), as the single-vector kernel
-    std::vector<int> groupFirst(G + 1, C);
-    for (int t = C - 1; t >= 0; --t) groupFirst[chunkGroup[t]] = t;
-    for (int g = G - 1; g >= 0; --g) groupFirst[g] = std::min(groupFirst[g], groupFirst[g + 1]);
-    const int stride = e.mpkStride == 1 ? 1 : 2;
-    for (int st = 0; st < G + stride * (power - 1); ++st)
-        for (int k = 0; k < power; ++k) {
-            const int g = st - stride * k;
-            if (g < 0 || g >= G) continue;
-            for (int t = groupFirst[g]; t < groupFirst[g + 1]; ++t) {
-                plan->itemChunk.push_back(t);
-                plan->itemPow.push_back((unsigned char)k);
-            }
-        }
     buildBatchTables(plan->tables, {plan.get()}, e.stream);
     return plan;
 }
@@ -330,8 +398,7 @@ void runBatch(BatchTables &t, cudaStream_t s) {
     RACE_CUDA(cudaMemsetAsync(t.ticket.p, 0, sizeof(int), s));
     RACE_CUDA(cudaMemsetAsync(t.status.p, 0, sizeof(int), s));
     if (t.numItems == 0) return;
-    BlockArgs a{t.members.p, t.chunkMember.p, t.chunkRow.p, t.chunkEnd.p, t.depRange.p, t.itemChunk.p,
-                t.itemPow.p, t.numItems, t.numChunks, t.done.p, t.ticket.p, t.status.p};
+    BlockArgs a{t.members.p, t.item.p, t.numItems, t.numChunks, t.done.p, t.ticket.p, t.status.p};
     dispatch<LaunchBlockFn>(t.valType, t.vecType, t.nrhs, a, s);
     RACE_CUDA(cudaGetLastError());
 }

@@ -103,10 +103,7 @@ struct BatchTables {
     int valType = 0, vecType = 0, nrhs = 1, maxPower = 0;
     int numChunks = 0, numItems = 0, numMembers = 0;
     DevBuf<BlockMember> members;
-    DevBuf<int> chunkMember, chunkRow, chunkEnd;  // numChunks each (local rows)
-    DevBuf<int> depRange;                          // numChunks*6, global chunk ids
-    DevBuf<int> itemChunk;                         // numItems
-    DevBuf<unsigned char> itemPow;                 // numItems
+    DevBuf<int4> item;                             // 3 per item, in issue order (batch.cu BlockArgs)
     DevBuf<int> done;                              // maxPower * numChunks
     DevBuf<int> ticket, status;
 };
@@ -118,8 +115,7 @@ struct BlockPlan {
     race_operands ops{};
     std::vector<int> chunkRow;   // numChunks+1
     std::vector<int> depRange;   // numChunks*6 (local chunk ids, empty range [0,-1])
-    std::vector<int> itemChunk;  // wavefront order
-    std::vector<unsigned char> itemPow;
+    std::vector<int> chunkGroup; // numChunks: level group
     BatchTables tables;
 };
 
