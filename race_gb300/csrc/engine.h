@@ -50,6 +50,7 @@ struct MpkPlan {
     int hubBig = 0, hubWork = 0;
     DevBuf<int> hubWorkRow, hubSegFirst, hubCount;
     DevBuf<double> hubSegPart;
+    DevBuf<float> hubBigVal;    // FP32/BF16: values of the rows that a block sums
     DevBuf<unsigned char> sellVal;  // sellSlots values (type valType)
     DevBuf<int> sellCol;        // sellSlots column indices (32-bit layout)
     // 16-bit layout (col16): per chunk four column window bases, per slot a

@@ -69,9 +69,9 @@ template <typename VT>
 constexpr int kSpmvMinBlocks = sizeof(VT) == 8 ? 0 : 8;
 constexpr int kSmallWarpsPerSm = 32;
 // Hub rows of FP32/BF16 values above this length are summed by a block each
-// (two tiles). The longest row bounds a power-law matrix, so the line hardly
-// matters: 151-153 us at 512 to 8,192 for the graph below.
-constexpr int kHubBlockLen = 4096;
+// (two tiles at least). The longest row bounds a power-law matrix, so the line
+// hardly matters: 110 and 116 us at 1,024 and 4,096 for the graph below.
+constexpr int kHubBlockLen = 1024;
 
 namespace {
 
@@ -154,14 +154,22 @@ struct SellView {
 // The hub rows as work of the plain SpMV. FP64: `num` segments of kMpkHubSeg
 // entries, a warp each (hub: the row of each; first: a row's first segment;
 // count: segments finished, zero between launches; part: their sums). FP32 and
-// BF16 values: the rows by falling length (hub), the first `big` a block each,
-// the `num` others a warp each.
+// BF16 values: the rows by falling length (hub), the first `big` a block each
+// (bigVal: their values in FP32, first: where each begins there), the `num`
+// others a warp each.
 struct HubWork {
     int big, num;
     const int *hub, *first;
     int *count;
     void *part;
+    const float *bigVal;
 };
+
+// Element offset of entry j of a lane's row inside its chunk: entries in
+// groups of four consecutive slots per lane (SELL-32 with 4-entry groups).
+__device__ __forceinline__ long long sellSlot(int j, int lane) {
+    return 32LL * (j & ~3) + 4 * lane + (j & 3);
+}
 
 // Vector loads of one entry group (four consecutive entries of a lane's
 // row), with an L2 policy (POL) or plain.
@@ -504,39 +512,43 @@ __global__ void __launch_bounds__(kWarpThreads, kMpkMinBlocks) kMpk(MpkArgs a) {
 __device__ __forceinline__ void pdlTrigger() { asm volatile("griddepcontrol.launch_dependents;"); }
 __device__ __forceinline__ void pdlWait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// One row as sellRowAcc, the matrix read one entry group ahead of the
-// gathers of x, its first group before x may be read at all.
+// One row as sellRowAcc, its columns read two entry groups ahead of the chain
+// and its values and x one, the first group's columns and values before x may
+// be read at all.
 template <typename VT, typename AT, bool C16>
 __device__ __forceinline__ AT sellRowAhead(const VT *__restrict__ val, long long voff, const void *col, long long coff,
                                            int4 b, int len, const AT *x) {
-    AT t = AT(0), v[4] = {AT(0), AT(0), AT(0), AT(0)};
-    int4 c = make_int4(0, 0, 0, 0);
+    AT t = AT(0), v[4] = {AT(0), AT(0), AT(0), AT(0)}, xv[4] = {AT(0), AT(0), AT(0), AT(0)};
+    int4 c = make_int4(0, 0, 0, 0), cn = c;
+    auto gather = [&](const int4 &q, int left, AT (&w)[4]) {
+        if (left > 0) w[0] = x[q.x];
+        if (left > 1) w[1] = x[q.y];
+        if (left > 2) w[2] = x[q.z];
+        if (left > 3) w[3] = x[q.w];
+    };
     if (len > 0) {
         groupVals<false>(val, voff, v, 0);
         c = groupCols<C16, false>(col, coff, b, 0);
     }
+    if (len > 4) cn = groupCols<C16, false>(col, coff + 128, b, 0);
     pdlWait();
+    gather(c, len, xv);
     for (int j = 0; j < len; j += 4) {
-        AT vn[4] = {AT(0), AT(0), AT(0), AT(0)};
-        int4 cn = make_int4(0, 0, 0, 0);
+        AT vn[4] = {AT(0), AT(0), AT(0), AT(0)}, xn[4] = {AT(0), AT(0), AT(0), AT(0)};
         if (j + 4 < len) {
+            gather(cn, len - j - 4, xn);
             groupVals<false>(val, voff + 32LL * (j + 4), vn, 0);
-            cn = groupCols<C16, false>(col, coff + 32LL * (j + 4), b, 0);
+            if (j + 8 < len) cn = groupCols<C16, false>(col, coff + 32LL * (j + 8), b, 0);
         }
-        if (len - j >= 4) {
-            const AT x0 = x[c.x], x1 = x[c.y], x2 = x[c.z], x3 = x[c.w];
-            t = fma(v[0], x0, t);
-            t = fma(v[1], x1, t);
-            t = fma(v[2], x2, t);
-            t = fma(v[3], x3, t);
-        } else {
-            t = fma(v[0], x[c.x], t);
-            if (len - j > 1) t = fma(v[1], x[c.y], t);
-            if (len - j > 2) t = fma(v[2], x[c.z], t);
-        }
+        t = fma(v[0], xv[0], t);
+        if (len - j > 1) t = fma(v[1], xv[1], t);
+        if (len - j > 2) t = fma(v[2], xv[2], t);
+        if (len - j > 3) t = fma(v[3], xv[3], t);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) v[q] = vn[q];
-        c = cn;
+        for (int q = 0; q < 4; ++q) {
+            v[q] = vn[q];
+            xv[q] = xn[q];
+        }
     }
     return t;
 }
@@ -586,86 +598,115 @@ __device__ __forceinline__ void hubTask(const SellView &m, const HubWork &hw, in
     }
 }
 
-// One long hub row (FP32/BF16) by a block: all warps gather the entries, a
-// tile of (value, x) pairs at a time, and the first runs hubSegment's 32
-// chains over the tiles, in its order. A warp alone waits for a round trip per
-// few entries of each lane; here the next tile's gathers and the columns of
-// the one after are in flight while a tile is summed.
-constexpr int kHubTile = 8 * kWarpThreads;  // entries: 16 KB of pairs
+// One long hub row (FP32/BF16) by a block: seven warps gather the entries, in
+// tiles of values and x, and the eighth runs hubSegment's 32 chains over the
+// tiles, in its order. A warp alone waits for a round trip per few entries of
+// each lane; here asynchronous copies bring three tiles ahead of the one being
+// summed, and the columns of three more are on their way.
+constexpr int kHubLoaders = kWarpThreads - 32;
+constexpr int kHubTile = 4 * kHubLoaders, kHubStages = 4;  // 28 entries a lane; 28 KB of pairs
 template <typename VT>
-__device__ __forceinline__ void hubBlock(const SellView &m, int h, int k, int n, const float *xin, double *x,
-                                         float *xf) {
-    __shared__ float2 tile[kHubTile];
-    constexpr int E = kHubTile / kWarpThreads;
-    const int beg = m.hubPtr[h], end = m.hubPtr[h + 1], tid = threadIdx.x;
-    const VT *__restrict__ val = (const VT *)m.hubVal;
-    int c[E];
-    float v[E], vn[E], xv[E];
-    auto load = [&](int t0, float (&w)[E]) {  // values and columns of the tile at t0
+__device__ __forceinline__ void hubBlock(const SellView &m, int h, const float *bigVal, int k, int n, const float *xin,
+                                         double *x, float *xf) {
+    __shared__ float sv[kHubStages][kHubTile], sx[kHubStages][kHubTile];
+    constexpr int E = kHubTile / kHubLoaders, A = kHubStages - 1, S = kHubTile / 32;
+    const int beg = m.hubPtr[h], len = m.hubPtr[h + 1] - beg;
+    const int tiles = (len + kHubTile - 1) / kHubTile;
+    if (threadIdx.x < 32) {
+        float t = 0.f;
+        for (int tile = 0; tile < tiles; ++tile) {
+            __syncthreads();  // the tile is there, and its stage's reuse waits for the next one
+            const float *v = sv[tile % kHubStages] + threadIdx.x, *xv = sx[tile % kHubStages] + threadIdx.x;
+            const int left = len - tile * kHubTile;
+            if (left >= kHubTile) {
 #pragma unroll
-        for (int i = 0; i < E; ++i) {
-            const int e = t0 + i * kWarpThreads + tid;
-            w[i] = e < end ? toF<VT>(val[e]) : 0.f;
-            c[i] = e < end ? m.hubCol[e] : -1;
+                for (int i = 0; i < S; ++i) t = fmaf(v[32 * i], xv[32 * i], t);
+            } else {
+                for (int i = 0; 32 * i + (int)threadIdx.x < left; ++i) t = fmaf(v[32 * i], xv[32 * i], t);
+            }
         }
-    };
-    auto gather = [&] {
-#pragma unroll
-        for (int i = 0; i < E; ++i) xv[i] = c[i] >= 0 ? xin[c[i]] : 0.f;
-    };
-    load(beg, v);
-    pdlWait();
-    gather();
-    load(beg + kHubTile, vn);
-    float t = 0.f;
-    for (int t0 = beg; t0 < end; t0 += kHubTile) {
-#pragma unroll
-        for (int i = 0; i < E; ++i) tile[i * kWarpThreads + tid] = make_float2(v[i], xv[i]);
-        __syncthreads();
-        gather();
-#pragma unroll
-        for (int i = 0; i < E; ++i) v[i] = vn[i];
-        load(t0 + 2 * kHubTile, vn);
-        if (tid < 32) {
-            const int cnt = min(kHubTile, end - t0);
-#pragma unroll 8
-            for (int i = tid; i < cnt; i += 32) t = fmaf(tile[i].x, tile[i].y, t);
-        }
-        __syncthreads();
-    }
-    if (tid < 32) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-        if (tid == 0) putRow(t, m.hubRow[h], k, n, x, xf);
+        if (threadIdx.x == 0) putRow(t, m.hubRow[h], k, n, x, xf);
+        return;
     }
+    const int id = threadIdx.x - 32;
+    const int *col = m.hubCol + beg;
+    int c[A][E];
+    auto columns = [&](int tile, int (&w)[E]) {
+#pragma unroll
+        for (int i = 0; i < E; ++i) {
+            const int e = tile * kHubTile + i * kHubLoaders + id;
+            w[i] = e < len ? col[e] : -1;
+        }
+    };
+    auto fetch = [&](int tile, const int (&w)[E]) {
+        const int st = tile % kHubStages;
+#pragma unroll
+        for (int i = 0; i < E; ++i) {
+            const int at = i * kHubLoaders + id;
+            if (w[i] < 0) continue;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
+                             (unsigned)__cvta_generic_to_shared(&sv[st][at])),
+                         "l"(bigVal + tile * kHubTile + at)
+                         : "memory");
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
+                             (unsigned)__cvta_generic_to_shared(&sx[st][at])),
+                         "l"(xin + w[i])
+                         : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int t = 0; t < A; ++t) columns(t, c[t]);
+    pdlWait();
+#pragma unroll
+    for (int t = 0; t < A; ++t) {
+        fetch(t, c[t]);
+        columns(t + A, c[t]);
+    }
+    for (int t0 = 0; t0 < tiles; t0 += A)
+#pragma unroll
+        for (int u = 0; u < A; ++u) {
+            const int tile = t0 + u;
+            if (tile >= tiles) break;
+            asm volatile("cp.async.wait_group %0;" ::"n"(A - 1) : "memory");  // this tile's copies
+            __syncthreads();  // everyone's, and the tile before is summed: its stage is free
+            fetch(tile + A, c[u]);
+            columns(tile + 2 * A, c[u]);
+        }
 }
 
-// Plain x_{k+1} = A x_k on the SELL layout, no schedule: one warp per hub
-// segment (they come first: the longest work) and per chunk. The next power's
-// launch overlaps this one's tail (pdlTrigger), which took 2-3 us a power:
-// 27-point 97x113x89, FP32, p = 8 (loads of 162 MB a power): 347 us before,
-// 305 us now; 7-point 32^3, FP64, p = 4 (launches): 25.3 and 14.3 us; BF16,
-// 150k-row power-law graph, p = 4: 790 us with one warp per hub row (rows of
-// up to 80k entries), 152-179 us now.
+// Plain x_{k+1} = A x_k on the SELL layout, no schedule: one warp per chunk,
+// and per hub row or segment (they come first: the longest work). The next
+// power's launch overlaps this one's tail (pdlTrigger), which took 2-3 us a
+// power. Measured on GB300, before all of this and now: 7-point 32^3, FP64,
+// p = 4 (launches): 25.3 and 11.9 us; BF16, 150k-row power-law graph, p = 4: 790
+// us with one warp per hub row (rows of up to 80k entries), 112 us; 27-point
+// 97x113x89, FP32, p = 8: 350 and 252 us; 7-point 110x101x107, FP64, p = 4: 119
+// and 92 us.
 //
-// kSpmvSell: a grid of resident warps striding the work, for matrices of
+// kSpmvSell: a grid of resident warps striding the chunks, for matrices of
 // several chunks a warp, where loads in flight (occupancy) decide: FP32 runs
-// with 32 registers and 8 blocks an SM.
+// with 32 registers and 8 blocks an SM. Odd powers run from the last chunk to
+// the first: what the L2 still holds of a matrix that does not fit is its end
+// (27-point 97x113x89, FP32: 162 MB a power, 305 us with all powers forward).
 template <typename VT, bool C16>
 __global__ void __launch_bounds__(kWarpThreads, kSpmvMinBlocks<VT>)
     kSpmvSell(SellView m, int numChunks, int n, int k, double *x, float *xf) {
     pdlTrigger();
     pdlWait();
     const int nw = gridDim.x * (blockDim.x >> 5);
-    for (int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < numChunks; c += nw)
-        chunkRow<VT, false, C16>(m, c, k, n, x, xf, 0);
+    for (int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < numChunks; i += nw)
+        chunkRow<VT, false, C16>(m, k & 1 ? numChunks - 1 - i : i, k, n, x, xf, 0);
 }
 
 // kSpmvSellSmall: one piece of work a warp, for matrices of at most
 // kSmallWarpsPerSm chunks an SM and those with hub rows, where the chain of
-// loads of a single row decides: row tables and first entry group are read
-// before the previous power is complete, later groups one ahead of their
-// gathers, hub rows with eight gathers a lane in flight.
+// loads of a single row decides: row tables and first entry groups are read
+// before the previous power is complete, later groups ahead of their chain
+// (7-point 32^3: 13.7 us with only the matrix ahead, 11.9 us with x ahead too),
+// hub rows with eight gathers a lane in flight.
 template <typename VT, bool HUBS, bool C16>
 __global__ void __launch_bounds__(kWarpThreads, kSmallWarpsPerSm * 32 / kWarpThreads)
     kSpmvSellSmall(SellView m, HubWork hw, int numChunks, int n, int k, double *x, float *xf) {
@@ -678,7 +719,7 @@ __global__ void __launch_bounds__(kWarpThreads, kSmallWarpsPerSm * 32 / kWarpThr
     if constexpr (HUBS) {
         if constexpr (sizeof(VT) != 8) {
             if ((int)blockIdx.x < hw.big) {
-                hubBlock<VT>(m, hw.hub[blockIdx.x], k, n, xin, x, xf);
+                hubBlock<VT>(m, hw.hub[blockIdx.x], hw.bigVal + hw.first[blockIdx.x], k, n, xin, x, xf);
                 return;
             }
             c -= hw.big * (kWarpThreads / 32);
@@ -753,10 +794,12 @@ __global__ void kGatherHubs(const int *__restrict__ rowPtr, const int *__restric
     }
 }
 
-// Element offset of entry j of a lane's row inside its chunk: entries in
-// groups of four consecutive slots per lane (SELL-32 with 4-entry groups).
-__device__ __forceinline__ long long sellSlot(int j, int lane) {
-    return 32LL * (j & ~3) + 4 * lane + (j & 3);
+// FP32 copies of the long hub rows' values, a block per row.
+template <typename VT>
+__global__ void kBigHubValues(const int *__restrict__ hub, const int *__restrict__ hubPtr, const VT *__restrict__ hval,
+                              const int *__restrict__ first, float *__restrict__ out) {
+    const int h = hub[blockIdx.x], beg = hubPtr[h], len = hubPtr[h + 1] - beg;
+    for (int j = threadIdx.x; j < len; j += blockDim.x) out[first[blockIdx.x] + j] = toF<VT>(hval[beg + j]);
 }
 
 // CRS -> SELL-32 copy; padding slots get value 0 and the row's own column.
@@ -937,6 +980,10 @@ void copySell(const race_operands &ops, MpkPlan &p, const int *chunkLen, cudaStr
     if (H)
         kGatherHubs<VT><<<ceilDiv(H, 8), 256, 0, s>>>(ops.rowPtr, ops.col, (const VT *)ops.val, p.hubRow.p,
                                                       p.hubPtr.p, H, (VT *)p.hubVal.p, p.hubCol.p);
+    if constexpr (sizeof(VT) != 8)
+        if (p.hubBig)
+            kBigHubValues<VT><<<p.hubBig, 256, 0, s>>>(p.hubWorkRow.p, p.hubPtr.p, (const VT *)p.hubVal.p,
+                                                       p.hubSegFirst.p, p.hubBigVal.p);
     RACE_CUDA(cudaGetLastError());
 }
 
@@ -1002,14 +1049,20 @@ std::unique_ptr<MpkPlan> buildMpkPlan(Engine &e, const race_operands &ops, int p
         }
         if (ops.val_type != RACE_VAL_F64) {
             std::stable_sort(work.begin(), work.end(), [&](int a, int b) { return hubLen(a) > hubLen(b); });
-            while (plan->hubBig < H && hubLen(work[plan->hubBig]) > kHubBlockLen) ++plan->hubBig;
+            segFirst.assign(1, 0);
+            for (; plan->hubBig < H && hubLen(work[plan->hubBig]) > kHubBlockLen; ++plan->hubBig)
+                segFirst.push_back(segFirst.back() + hubLen(work[plan->hubBig]));
         }
         plan->hubWork = (int)work.size() - plan->hubBig;
         plan->hubWorkRow.upload(work.data(), work.size(), s);
         plan->hubSegFirst.upload(segFirst.data(), segFirst.size(), s);
-        plan->hubSegPart.alloc(segFirst.back());
-        plan->hubCount.alloc(H);
-        RACE_CUDA(cudaMemsetAsync(plan->hubCount.p, 0, sizeof(int) * H, s));
+        if (ops.val_type == RACE_VAL_F64) {
+            plan->hubSegPart.alloc(segFirst.back());
+            plan->hubCount.alloc(H);
+            RACE_CUDA(cudaMemsetAsync(plan->hubCount.p, 0, sizeof(int) * H, s));
+        } else {
+            plan->hubBigVal.alloc(std::max(segFirst.back(), 1));
+        }
         RACE_CUDA(cudaStreamSynchronize(s));  // work and segFirst go out of scope
     }
     plan->numChunks = C;
@@ -1253,7 +1306,7 @@ void launchSpmvSellK(const MpkPlan &p, int n, int k, double *x, cudaStream_t s) 
     cfg.numAttrs = 1;
     const int blocks = std::max(1, ceilDiv((long long)p.hubWork + p.numChunks, kWarpThreads / 32));
     if (HUBS || p.numChunks <= kSmallWarpsPerSm * devSms()) {
-        const HubWork hw{p.hubBig, p.hubWork, p.hubWorkRow.p, p.hubSegFirst.p, p.hubCount.p, p.hubSegPart.p};
+        const HubWork hw{p.hubBig, p.hubWork, p.hubWorkRow.p, p.hubSegFirst.p, p.hubCount.p, p.hubSegPart.p, p.hubBigVal.p};
         cfg.gridDim = dim3(p.hubBig + blocks);
         RACE_CUDA(cudaLaunchKernelEx(&cfg, kSpmvSellSmall<VT, HUBS, C16>, viewOf(p), hw, p.numChunks, n, k, x, p.xf.p));
         return;
