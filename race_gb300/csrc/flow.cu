@@ -32,12 +32,12 @@
 // is an L2 store and a load that sees it (850-1100 cycles), the row's FP64
 // chain (a warp's FP64 instruction occupies its quarter of the SM for 64
 // cycles, whether 1 or 32 lanes are active) and an FP64 division (570
-// cycles), about 1.5 us in all. The wave executor took 5.7 us a wave (a grid
+// cycles), about 1.4 us in all. The wave executor took 5.7 us a wave (a grid
 // barrier of 152 blocks is 1.25 us, the row data loaded after it the rest),
 // the leaf executor one serial row after another in each leaf. Forward +
 // backward sweeps, before and after: Gauss-Seidel, 27-point 40x44x41 (leaf
-// sums, 248 waves a direction), FP64 2450 and 770 us; Kaczmarz, 9-point
-// 211x197 (leaf sums, 181 waves) 1150 and 556 us; the refinement solve of a
+// sums, 248 waves a direction), FP64 2450 and 692 us; Kaczmarz, 9-point
+// 211x197 (leaf sums, 181 waves) 1150 and 511 us; the refinement solve of a
 // 100k-row power-law graph (sequential sums, FP32, 24 refinements of two
 // sweeps of 315 waves) 100 and 19.6 ms.
 #include <algorithm>
@@ -51,8 +51,8 @@ namespace {
 
 // One block of 8 warps per SM: 1,216 tasks (of up to 4 or 32 rows) in flight,
 // several waves of an ordinary matrix, so that a task's row data is loaded
-// before its inputs arrive (4 warps: 787 us for the 770 us above, 16: 890,
-// whose polling slows the running rows).
+// before its inputs arrive. 4 warps took 2 % more time on the Gauss-Seidel
+// pair above, 16 took 16 % more: their polling slows the running rows.
 constexpr int kFlowThreads = 256;
 constexpr int kFlowWarps = kFlowThreads / 32;
 
@@ -254,7 +254,7 @@ __device__ __forceinline__ bool chunkTask(const FlowArgs &a, const int4 &t, int 
     const int len = live ? q.z : 0;
     const int most = __reduce_max_sync(0xffffffffu, len);
     const long long off = a.chunkOff ? a.chunkOff[t.w] : -1;
-    const XT br = live ? ((const XT *)a.b)[r] : XT(0);
+    const XT br = live ? ((const XT *)a.b)[r] : XT(1);  // idle lanes divide 1 by 1 (see lanesTask)
     XT v[kBlk], xv[kBlk];
     int c[kBlk], m[kBlk];
     unsigned valid = 0;
@@ -403,7 +403,10 @@ __device__ __forceinline__ bool lanesTask(const FlowArgs &a, const int4 &t, int 
     const int4 q = live ? a.pos[t.y + sub] : make_int4(0, 0, 0, 0);
     const int r = q.x, s = q.y, e = q.y + q.z;
     const VT *val = (const VT *)a.val;
-    const XT br = live ? ((const XT *)a.b)[r] : XT(0);
+    // Idle lanes divide 1 by 1: a zero numerator sends the whole warp through
+    // the FP64 division's special cases (775 us instead of 692 us for the
+    // Gauss-Seidel pair above, 559 instead of 511 us for the Kaczmarz pair).
+    const XT br = live ? ((const XT *)a.b)[r] : XT(1);
     XT diag = XT(1), v[E], xv[E], p[E];
     if constexpr (!KACZ)
         if (e > s) diag = ld<VT, XT>(val, s);
