@@ -6,18 +6,20 @@
 // are one flat array: for each layer W then b. The tuner's network is small
 // (34 inputs, 3 x 128 hidden, 1 output) and its batches are some hundreds to
 // thousands of rows: a product is a few million multiply-adds, so launches and
-// the latency of each bound the time, not arithmetic. The whole forward pass
-// is therefore one kernel (kForward: a block takes a few rows through all
-// layers, activations in shared memory, weights in tiles fetched one ahead
-// across the layer boundaries), the loss and the data gradients another
-// (kBackward) and all layers' weight and bias gradients a third (kWeightGrad).
-// One kernel per product took 16 launches: loss and gradients of 239 rows
-// were 146 us on the GPU (222 us a call), one 32 x 32 tile after another for
-// the weight gradients and one thread per column for the bias sums; now 32 us
-// in three launches (77 us a call, the rest is the gradients' way to the
-// caller's host memory).
-// Networks wider than kFusedDim or deeper than kFusedLayers run the products
-// one by one (kGemm: 32 x 32 output tiles, 16-deep k slices).
+// the latency of each bound the time, not arithmetic. Forward pass and data
+// gradients are therefore one kernel that holds the whole network in shared
+// memory (kResident), all layers' weight and bias gradients and the loss
+// another (kWeightGrad), which writes the caller's copy as well. Loss and
+// gradients of 239 rows, on the GPU and per call: one kernel per product (16
+// launches) 146 and 222 us; forward and backward kernels that fetch the weights
+// tile by tile and 32 x 32 gradient tiles 33 and 77 us; now 18.5 and 47 us
+// (512 rows 83 -> 54, 4,096: 131 -> 100, 65,536: 1,179 -> 883). Outputs alone,
+// 239 rows: 14.4 -> 10.3 us.
+// Networks that do not fit in shared memory take the tiles (kForward: a block
+// takes a few rows through all layers, weights in tiles fetched one ahead
+// across the layer boundaries; kBackward), networks wider than kFusedDim or
+// deeper than kFusedLayers the products one by one (kGemm: 32 x 32 output
+// tiles, 16-deep k slices).
 // Each output sums its terms in order with fmaf in either form, so results do
 // not depend on the grid; above kGradRows rows the weight gradients are summed
 // in chunks of rows, added in order (kGradReduce). The loss reduction runs in
@@ -124,6 +126,8 @@ constexpr int kFusedDim = 1024;   // widest layer: the rows of two layers fit in
 // mean fewer of them.
 constexpr int kTileN = 128, kTileK = 64, kTileVals = kTileN * kTileK / 256;
 constexpr size_t kTileBytes = 2 * sizeof(float) * kTileK * (kTileN + 1);
+constexpr size_t kResidentBytes = 227 * 1024;  // shared memory of one block, all of it
+constexpr int kResidentSms = 152;
 constexpr int kGradRows = 512;    // rows summed in one chain per weight gradient
 constexpr int kGradChunk = 256;   // rows of a chunk beyond that (at most kGradChunks chunks)
 constexpr int kGradChunks = 64;
@@ -254,30 +258,15 @@ __global__ void __launch_bounds__(256) kForward(NetView v, const float *__restri
 }
 
 // Output gradients 2 (y - t) / (B O), then the data gradients of all layers
-// for R rows; block 0 also reduces the loss as kMse does.
+// for R rows.
 template <int R>
-__global__ void __launch_bounds__(256) kBackward(NetView v, const float *__restrict__ T, int B, int D, float *loss) {
+__global__ void __launch_bounds__(256) kBackward(NetView v, const float *__restrict__ T, int B, int D) {
     extern __shared__ __align__(16) float smem[];
     auto sw = (float(*)[kTileK][kTileN + 1]) smem;
     float *sx = smem + kTileBytes / sizeof(float);
     const int m0 = blockIdx.x * R, last = v.layers - 1, out = v.dimOut[last], count = B * out;
     const float *y = v.act[last];
     const float scale = 2.f / (float)count;
-    if (blockIdx.x == 0) {
-        __shared__ float part[256];
-        float s = 0.f;
-        for (int i = threadIdx.x; i < count; i += 256) {
-            const float d = y[i] - T[i];
-            s = fmaf(d, d, s);
-        }
-        part[threadIdx.x] = s;
-        __syncthreads();
-        for (int w = 128; w > 0; w >>= 1) {
-            if (threadIdx.x < w) part[threadIdx.x] += part[threadIdx.x + w];
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) *loss = part[0] / (float)count;
-    }
     for (int i = threadIdx.x; i < R * out; i += 256) {
         const int r = i / out, n = i % out;
         const size_t o = (size_t)(m0 + r) * out + n;
@@ -295,57 +284,302 @@ __global__ void __launch_bounds__(256) kBackward(NetView v, const float *__restr
     });
 }
 
-// Weight and bias gradients of every layer, one 32 x 32 tile of one layer a
-// block (grid.x) over rows [chunk * rows, ...) (grid.y): dW[n][k] = sum of
-// delta[m][n] x[m][k], db[n] = sum of delta[m][n], in order of m. One chunk
-// writes the gradients, more write their own copies (part + chunk * stride).
-constexpr int kGradTile = 32, kGradSlice = 32;
-__global__ void __launch_bounds__(256) kWeightGrad(NetView v, const float *__restrict__ X, int B, int rows,
-                                                   const float *gradBase, float *part, size_t stride) {
-    __shared__ float sd[2][kGradSlice][kGradTile + 1], sx[2][kGradSlice][kGradTile + 1];
+// 4- and 16-byte asynchronous copies to shared memory; !on writes zeros.
+__device__ __forceinline__ void copy4(float *dst, const float *src, bool on) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
+                 "r"(on ? 4 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void copy16(float *dst, const float *src, bool on) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(on ? 16 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void copyCommit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// At most `left` of the latest groups may still be on their way (3 and more count as 3).
+__device__ __forceinline__ void copyWait(int left) {
+    if (left >= 3) asm volatile("cp.async.wait_group 3;" ::: "memory");
+    else if (left == 2) asm volatile("cp.async.wait_group 2;" ::: "memory");
+    else if (left == 1) asm volatile("cp.async.wait_group 1;" ::: "memory");
+    else asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
+// Floats between two rows of a layer's weights in shared memory: whole
+// float4s, an odd number of them, so that neither a warp reading one float4
+// of 32 rows (forward) nor 32 values of one row (backward) meets a bank twice
+// in a quarter.
+__host__ __device__ inline int weightStride(int K) { return 4 * (((K + 3) / 4) | 1); }
+__host__ __device__ inline int layerFloats(int K, int N) { return N * weightStride(K) + ((N + 3) & ~3); }
+
+// acc[i] += sum of x[i][k] w(k..k+3) over whole groups of four terms, in
+// order; returns the number of terms. Sixteen terms' operands are read before
+// the first multiply-add (8 and 4 where a thread has more rows, which hide the
+// reads): 128 terms of one result took 2,450 cycles four at a time, 800 so.
+// A float4 that the whole warp reads costs shared memory as much as 32
+// different ones, so fewer rows a block are faster while they fit on the GPU.
+template <int H, typename W>
+__device__ __forceinline__ int termSums(float (&acc)[H], const float *x, int D, int K, W &&weight) {
+    constexpr int S = H <= 2 ? 4 : H <= 4 ? 2 : 1;
+    int k = 0;
+    auto some = [&](auto groups) {
+        constexpr int G = decltype(groups)::value;
+        float4 w[G], q[G][H];
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            w[g] = weight(k + 4 * g);
+#pragma unroll
+            for (int i = 0; i < H; ++i) q[g][i] = *(const float4 *)(x + i * D + k + 4 * g);
+        }
+#pragma unroll
+        for (int g = 0; g < G; ++g)
+#pragma unroll
+            for (int i = 0; i < H; ++i)
+                acc[i] = fmaf(q[g][i].w, w[g].w,
+                              fmaf(q[g][i].z, w[g].z, fmaf(q[g][i].y, w[g].y, fmaf(q[g][i].x, w[g].x, acc[i]))));
+        k += 4 * G;
+    };
+    while (k + 4 * S <= K) some(std::integral_constant<int, S>{});
+    while (k + 4 <= K) some(std::integral_constant<int, 1>{});
+    return k;
+}
+
+// All layers of R rows at a time with every weight of the network in shared
+// memory: forward, and for TRAIN the output gradients 2 (y - t) / (B O) and
+// the data gradients of all layers behind it. The weights are copied once a
+// block, a layer a group, the sums of a layer wait for its group only;
+// forward and backward read the same copy (W[n][k] along k and along n). Rows
+// are taken in turns of the grid, so a network's weights are read once per
+// resident block. A tile at a time through registers (kForward, kBackward)
+// paid an L2 round trip and a barrier per tile, 14 of them for the tuner's
+// network: 12.3 + 9.6 us of 239 rows, here 11.4 (7,000 cycles for the copies,
+// 2,000 a layer, bound by shared memory: see termSums). Two columns a thread
+// in four warps measured the same, one latency after another.
+template <int R, bool TRAIN>
+__global__ void __launch_bounds__(256) kResident(NetView v, const float *__restrict__ X, const float *__restrict__ T,
+                                                 int B, int D, float *yOut) {
+    extern __shared__ __align__(16) float smem[];
+    constexpr int H = R / 2;
+    const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
+    const int col = threadIdx.x % 128, half = threadIdx.x / 128;
+    const int last = v.layers - 1, in = v.dimIn[0], out = v.dimOut[last];
+    int total = 0;
+    for (int l = 0; l < v.layers; ++l) {
+        const int K = v.dimIn[l], N = v.dimOut[l], ld = weightStride(K);
+        const float *w = v.w[l];
+        float *sw = smem + total;
+        if (K % 4 == 0 && ((size_t)w & 15) == 0) {
+            for (int k = 4 * lane; k < K; k += 128)
+                for (int m = warp; m < N; m += 64)
+#pragma unroll
+                    for (int n = m; n < m + 64; n += 8)
+                        if (n < N) copy16(sw + n * ld + k, w + n * K + k, true);
+        } else {
+            for (int k = lane; k < K; k += 32)
+                for (int m = warp; m < N; m += 64)
+#pragma unroll
+                    for (int n = m; n < m + 64; n += 8)
+                        if (n < N) copy4(sw + n * ld + k, w + n * K + k, true);
+        }
+        for (int n = threadIdx.x; n < N; n += 256) copy4(sw + N * ld + n, v.b[l] + n, true);
+        copyCommit();
+        total += layerFloats(K, N);
+    }
+    float *sx = smem + total;
+    const float scale = 2.f / (float)(B * out);
+    bool first = true;
+    for (int m0 = blockIdx.x * R; m0 < B; m0 += gridDim.x * R, first = false) {
+        int cur = 0, base = 0;
+        __syncthreads();  // the rows before are done with
+        for (int i = threadIdx.x; i < R * in; i += 256) {
+            const int r = i / in, k = i % in;
+            sx[(size_t)r * D + k] = m0 + r < B ? X[(size_t)(m0 + r) * in + k] : 0.f;
+        }
+        for (int l = 0; l < v.layers; ++l, cur ^= 1) {
+            const int K = v.dimIn[l], N = v.dimOut[l], ld = weightStride(K);
+            const float *sw = smem + base, *x = sx + (size_t)(cur * R + half * H) * D;
+            float *xn = sx + (size_t)((cur ^ 1) * R + half * H) * D;
+            if (first) copyWait(last - l);
+            __syncthreads();  // the layer's weights and rows
+            for (int n = col; n < N; n += 128) {
+                const float *wr = sw + n * ld;
+                float acc[H];
+#pragma unroll
+                for (int i = 0; i < H; ++i) acc[i] = 0.f;
+                const int k = termSums<H>(acc, x, D, K, [&](int k) { return *(const float4 *)(wr + k); });
+                for (int j = k; j < K; ++j)
+#pragma unroll
+                    for (int i = 0; i < H; ++i) acc[i] = fmaf(x[i * D + j], wr[j], acc[i]);
+                const float bias = sw[N * ld + n];
+#pragma unroll
+                for (int i = 0; i < H; ++i) {
+                    const int row = m0 + half * H + i;
+                    float s = acc[i] + bias;
+                    if (l < last) s = fmaxf(s, 0.f);
+                    xn[(size_t)i * D + n] = s;
+                    if (row >= B) continue;
+                    if (TRAIN) v.act[l][(size_t)row * N + n] = s;
+                    else if (l == last) yOut[(size_t)row * N + n] = s;
+                }
+            }
+            base += layerFloats(K, N);
+        }
+        if (!TRAIN) continue;
+        __syncthreads();
+        for (int i = threadIdx.x; i < R * out; i += 256) {
+            const int r = i / out, n = i % out;
+            const size_t o = (size_t)(m0 + r) * out + n;
+            float d = 0.f;
+            if (m0 + r < B) v.delta[last][o] = d = scale * (sx[(size_t)(cur * R + r) * D + n] - T[o]);
+            sx[(size_t)((cur ^ 1) * R + r) * D + n] = d;
+        }
+        cur ^= 1;
+        for (int l = last; l > 0; --l, cur ^= 1) {
+            const int K = v.dimOut[l], N = v.dimIn[l], ld = weightStride(N);
+            base -= layerFloats(N, K);
+            const float *sw = smem + base, *x = sx + (size_t)(cur * R + half * H) * D;
+            float *xn = sx + (size_t)((cur ^ 1) * R + half * H) * D;
+            __syncthreads();
+            for (int n = col; n < N; n += 128) {
+                float acc[H], act[H];  // act: this thread's own stores of the forward pass
+#pragma unroll
+                for (int i = 0; i < H; ++i) {
+                    const int row = m0 + half * H + i;
+                    acc[i] = 0.f;
+                    act[i] = row < B ? v.act[l - 1][(size_t)row * N + n] : 0.f;
+                }
+                const int k = termSums<H>(acc, x, D, K, [&](int k) {
+                    const float *wk = sw + k * ld + n;
+                    return make_float4(wk[0], wk[ld], wk[2 * ld], wk[3 * ld]);
+                });
+                for (int j = k; j < K; ++j)
+#pragma unroll
+                    for (int i = 0; i < H; ++i) acc[i] = fmaf(x[i * D + j], sw[j * ld + n], acc[i]);
+#pragma unroll
+                for (int i = 0; i < H; ++i) {
+                    const int row = m0 + half * H + i;
+                    const float s = row < B && act[i] > 0.f ? acc[i] : 0.f;
+                    if (row < B) v.delta[l - 1][(size_t)row * N + n] = s;
+                    xn[(size_t)i * D + n] = s;
+                }
+            }
+        }
+    }
+}
+
+// Weight and bias gradients of every layer, one tile of 4 NW outputs x 32 KW
+// inputs of one layer a block (grid.x) over rows [chunk * rows, ...) (grid.y):
+// dW[n][k] = sum of delta[m][n] x[m][k], db[n] = sum of delta[m][n], in order
+// of m. One chunk writes the gradients, more write their own copies (part +
+// chunk * stride). The block after the tiles reduces the loss as kMse does.
+// A thread holds NW outputs of KW inputs, which take NW + KW shared-memory
+// accesses a row (a value that the whole warp reads costs one too): 2 x 1
+// where one chain of rows leaves the GPU idle and the longest block counts, 4
+// x 2 for chunks of rows. Slices of 32 rows are copied three ahead. With host
+// (pinned memory) the gradients and the loss are written there too: a copy
+// behind the kernels cost 5 us a call.
+constexpr int kGradSlice = 32, kGradStages = 4;
+template <int NW, int KW>
+__global__ void __launch_bounds__(128) kWeightGrad(NetView v, const float *__restrict__ X, const float *__restrict__ T,
+                                                   int B, int rows, const float *gradBase, float *part, size_t stride,
+                                                   float *loss, float *host) {
+    constexpr int kGradN = 4 * NW, kGradK = 32 * KW;
+    __shared__ __align__(16) float sd[kGradStages][kGradSlice][kGradN];
+    __shared__ __align__(16) float sx[kGradStages][kGradSlice][kGradK];
+    // Set up while the pass before ends. It does not let this grid start
+    // earlier: blocks that wait crowd on the SMs that are free then and stay
+    // there (239 rows 24.6 us for both, so 18.5).
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (blockIdx.x == gridDim.x - 1) {
+        if (blockIdx.y) return;
+        float *sum = &sx[0][0][0];
+        const float *y = v.act[v.layers - 1];
+        const int count = B * v.dimOut[v.layers - 1];
+        float s[2] = {0.f, 0.f};
+        for (int i = threadIdx.x; i < count; i += 256)
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+                if (i + 128 * j < count) {
+                    const float d = y[i + 128 * j] - T[i + 128 * j];
+                    s[j] = fmaf(d, d, s[j]);
+                }
+        sum[threadIdx.x] = s[0] + s[1];
+        __syncthreads();
+        for (int w = 64; w > 0; w >>= 1) {
+            if (threadIdx.x < w) sum[threadIdx.x] += sum[threadIdx.x + w];
+            __syncthreads();
+        }
+        if (threadIdx.x == 0) {
+            *loss = sum[0] / (float)count;
+            if (host) host[loss - gradBase] = sum[0] / (float)count;
+        }
+        return;
+    }
     int l = 0, tile = blockIdx.x, tk = 0;
     for (;; ++l) {
-        tk = (v.dimIn[l] + kGradTile - 1) / kGradTile;
-        const int tiles = tk * ((v.dimOut[l] + kGradTile - 1) / kGradTile);
+        tk = (v.dimIn[l] + kGradK - 1) / kGradK;
+        const int tiles = tk * ((v.dimOut[l] + kGradN - 1) / kGradN);
         if (tile < tiles) break;
         tile -= tiles;
     }
     const int N = v.dimOut[l], K = v.dimIn[l];
-    const int n0 = (tile / tk) * kGradTile, k0 = (tile % tk) * kGradTile;
+    const int n0 = (tile / tk) * kGradN, k0 = (tile % tk) * kGradK;
     const float *d = v.delta[l], *x = l == 0 ? X : v.act[l - 1];
     const int m0 = blockIdx.y * rows, m1 = min(B, m0 + rows);
     const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    float rd[4], rx[4], acc[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, bias = 0.f;
-    auto load = [&](int m) {
+    const bool wide = K % 4 == 0 && ((size_t)x & 15) == 0;
+    auto load = [&](int m, int stage) {
+        if (m < m1) {
+            if (wide) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int row = m + warp + 8 * i;
-            rd[i] = row < m1 && n0 + lane < N ? d[(size_t)row * N + n0 + lane] : 0.f;
-            rx[i] = row < m1 && k0 + lane < K ? x[(size_t)row * K + k0 + lane] : 0.f;
+                for (int i = 0; i < 2 * KW; ++i) {
+                    const int e = threadIdx.x + 128 * i, q = e / (8 * KW), k = 4 * (e % (8 * KW));
+                    const bool on = m + q < m1 && k0 + k < K;
+                    copy16(&sx[stage][q][k], on ? x + (size_t)(m + q) * K + k0 + k : x, on);
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 8 * KW; ++i) {
+                    const int e = threadIdx.x + 128 * i, q = e / kGradK, k = e % kGradK;
+                    const bool on = m + q < m1 && k0 + k < K;
+                    copy4(&sx[stage][q][k], on ? x + (size_t)(m + q) * K + k0 + k : x, on);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < NW; ++i) {
+                const int e = threadIdx.x + 128 * i, q = e / kGradN, n = e % kGradN;
+                const bool on = m + q < m1 && n0 + n < N;
+                copy4(&sd[stage][q][n], on ? d + (size_t)(m + q) * N + n0 + n : d, on);
+            }
         }
+        copyCommit();
     };
-    load(m0);
-    int buf = 0;
-    for (int m = m0; m < m1; m += kGradSlice, buf ^= 1) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            sd[buf][warp + 8 * i][lane] = rd[i];
-            sx[buf][warp + 8 * i][lane] = rx[i];
-        }
-        __syncthreads();
-        if (m + kGradSlice < m1) load(m + kGradSlice);
+    for (int i = 0; i < kGradStages - 1; ++i) load(m0 + i * kGradSlice, i);
+    float acc[NW][KW] = {}, bias[NW] = {};
+    int stage = 0;
+    for (int m = m0; m < m1; m += kGradSlice, stage = (stage + 1) % kGradStages) {
+        copyWait(kGradStages - 2);
+        __syncthreads();  // this slice is there, and the one before is done with
+        load(m + (kGradStages - 1) * kGradSlice, (stage + kGradStages - 1) % kGradStages);
         const int end = min(kGradSlice, m1 - m);
-#pragma unroll 8
-        for (int q = 0; q < end; ++q) {
-            const float d0 = sd[buf][q][ty], d1 = sd[buf][q][ty + 16], x0 = sx[buf][q][tx], x1 = sx[buf][q][tx + 16];
-            acc[0][0] = fmaf(d0, x0, acc[0][0]);
-            acc[0][1] = fmaf(d0, x1, acc[0][1]);
-            acc[1][0] = fmaf(d1, x0, acc[1][0]);
-            acc[1][1] = fmaf(d1, x1, acc[1][1]);
+        auto step = [&](int q) {
+            float dn[NW], xk[KW];
+#pragma unroll
+            for (int j = 0; j < NW; ++j) dn[j] = sd[stage][q][NW * warp + j];
+#pragma unroll
+            for (int j = 0; j < KW; ++j) xk[j] = sx[stage][q][32 * j + lane];
+#pragma unroll
+            for (int j = 0; j < NW; ++j) {
+#pragma unroll
+                for (int i = 0; i < KW; ++i) acc[j][i] = fmaf(dn[j], xk[i], acc[j][i]);
+                bias[j] += dn[j];
+            }
+        };
+        if (end == kGradSlice) {
+#pragma unroll 16
+            for (int q = 0; q < kGradSlice; ++q) step(q);
+        } else {
+            for (int q = 0; q < end; ++q) step(q);
         }
-        if (k0 == 0 && warp == 0)
-            for (int q = 0; q < end; ++q) bias += sd[buf][q][lane];
     }
     float *dw = v.dw[l], *db = v.db[l];
     if (part) {
@@ -353,23 +587,32 @@ __global__ void __launch_bounds__(256) kWeightGrad(NetView v, const float *__res
         db = part + (size_t)blockIdx.y * stride + (db - gradBase);
     }
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+    for (int j = 0; j < NW; ++j) {
+        const int n = n0 + NW * warp + j;
+        if (n >= N) continue;
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const int n = n0 + ty + 16 * i, k = k0 + tx + 16 * j;
-            if (n < N && k < K) dw[(size_t)n * K + k] = acc[i][j];
+        for (int i = 0; i < KW; ++i) {
+            const int k = k0 + 32 * i + lane;
+            if (k >= K) continue;
+            dw[(size_t)n * K + k] = acc[j][i];
+            if (host && !part) host[dw - gradBase + (size_t)n * K + k] = acc[j][i];
         }
-    if (k0 == 0 && warp == 0 && n0 + lane < N) db[n0 + lane] = bias;
+        if (k0 == 0 && lane == 0) {
+            db[n] = bias[j];
+            if (host && !part) host[db - gradBase + n] = bias[j];
+        }
+    }
 }
 
 // Sum of the chunks' gradients, in order of the chunks.
 __global__ void __launch_bounds__(256) kGradReduce(long long n, int chunks, const float *__restrict__ part,
-                                                   size_t stride, float *__restrict__ grad) {
+                                                   size_t stride, float *__restrict__ grad, float *host) {
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (i >= n) return;
     float s = part[i];
     for (int c = 1; c < chunks; ++c) s += part[c * stride + i];
     grad[i] = s;
+    if (host) host[i] = s;
 }
 
 // Adam (Kingma & Ba 2015) with bias correction.
@@ -471,10 +714,10 @@ struct Mlp {
     // shared memory of R rows of two layers, the widest padded to whole float4
     int rowStride() const { return (std::max(in, std::max(hidden, out)) + 3) & ~3; }
     static int passBytes(int R, int stride) { return (int)(kTileBytes + 2 * R * stride * sizeof(float)); }
-    // Rows a block: 4 while that leaves at most one block an SM (239 rows: 60
-    // blocks), then 8, and 16 where enough blocks remain to share each weight
-    // tile among more rows.
-    static int rowsPerBlock(int B) { return B <= 4 * 152 ? 4 : B <= 8 * 152 ? 8 : 16; }
+    // Rows a block: 2 while that leaves at most one block an SM (239 rows: 120
+    // blocks, 18.5 us for loss and gradients, 4 rows 20.5), then 4 and 8, and 16
+    // where enough blocks remain to share each weight among more rows.
+    static int rowsPerBlock(int B) { return B <= 2 * 152 ? 2 : B <= 4 * 152 ? 4 : B <= 8 * 152 ? 8 : 16; }
     template <int R>
     void fusedForward(const NetView &v, const float *X, int B, float *y, cudaStream_t s) {
         static const cudaError_t opt = cudaFuncSetAttribute(
@@ -487,14 +730,34 @@ struct Mlp {
         static const cudaError_t opt = cudaFuncSetAttribute(
             kBackward<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, passBytes(R, kFusedDim));
         RACE_CUDA(opt);
-        kBackward<R><<<ceilDiv(B, R), 256, passBytes(R, rowStride()), s>>>(v, T, B, rowStride(), loss());
+        kBackward<R><<<ceilDiv(B, R), 256, passBytes(R, rowStride()), s>>>(v, T, B, rowStride());
+    }
+    // Shared memory of the whole network and R rows of two layers (164 KB for
+    // the tuner's network and 8 rows); where it fits, kResident takes the pass
+    // (239 rows, loss and gradients on the GPU: 33 us by tiles, 18.5 resident).
+    size_t residentBytes(int R) const {
+        size_t f = 2 * (size_t)R * rowStride();
+        for (int l = 0; l < layers(); ++l) f += layerFloats(dimIn[l], dimOut[l]);
+        return sizeof(float) * f;
+    }
+    template <int R, bool TRAIN>
+    bool residentPass(const NetView &v, const float *X, const float *T, int B, float *y, cudaStream_t s) {
+        const size_t bytes = residentBytes(R);
+        if (bytes > kResidentBytes) return false;
+        static const cudaError_t opt = cudaFuncSetAttribute(
+            kResident<R, TRAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResidentBytes);
+        RACE_CUDA(opt);
+        const int perSm = (int)std::max<size_t>(1, std::min<size_t>(8, kResidentBytes / (bytes + 1024)));
+        kResident<R, TRAIN><<<std::min(ceilDiv(B, R), kResidentSms * perSm), 256, bytes, s>>>(v, X, T, B, rowStride(), y);
+        return true;
     }
     template <typename F>
     void byRows(int B, F &&f) {
         switch (rowsPerBlock(B)) {
         case 16: f(std::integral_constant<int, 16>{}); break;
         case 8: f(std::integral_constant<int, 8>{}); break;
-        default: f(std::integral_constant<int, 4>{}); break;
+        case 4: f(std::integral_constant<int, 4>{}); break;
+        default: f(std::integral_constant<int, 2>{}); break;
         }
         RACE_CUDA(cudaGetLastError());
     }
@@ -506,26 +769,48 @@ struct Mlp {
             return;
         }
         const NetView v = view(0);
-        byRows(B, [&](auto r) { fusedForward<decltype(r)::value>(v, X, B, Y, s); });
+        byRows(B, [&](auto r) {
+            constexpr int R = decltype(r)::value;
+            if (!residentPass<R, false>(v, X, nullptr, B, Y, s)) fusedForward<R>(v, X, B, Y, s);
+        });
     }
-    void lossGradFused(const float *X, const float *T, int B, cudaStream_t s) {
+    template <int NW, int KW>
+    void weightGrad(const NetView &v, const float *X, const float *T, int B, int rows, int chunks, size_t stride,
+                    float *host, cudaStream_t s) {
+        int tiles = 0;
+        for (int l = 0; l < layers(); ++l) tiles += ceilDiv(dimOut[l], 4 * NW) * ceilDiv(dimIn[l], 32 * KW);
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(tiles + 1, chunks);
+        cfg.blockDim = dim3(128);
+        cfg.stream = s;
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeProgrammaticStreamSerialization;  // starts as the pass ends, waits for it
+        at.val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        RACE_CUDA(cudaLaunchKernelEx(&cfg, kWeightGrad<NW, KW>, v, X, T, B, rows, (const float *)grads.p,
+                                     chunks > 1 ? part.p : (float *)nullptr, stride, loss(), host));
+    }
+    void lossGradFused(const float *X, const float *T, int B, float *host, cudaStream_t s) {
         ensure(B);
         const NetView v = view(B);
-        byRows(B, [&](auto r) { fusedForward<decltype(r)::value>(v, X, B, nullptr, s); });
-        byRows(B, [&](auto r) { fusedBackward<decltype(r)::value>(v, T, B, s); });
-        int tiles = 0;
-        for (int l = 0; l < layers(); ++l) tiles += ceilDiv(dimOut[l], kGradTile) * ceilDiv(dimIn[l], kGradTile);
+        byRows(B, [&](auto r) {
+            constexpr int R = decltype(r)::value;
+            if (residentPass<R, true>(v, X, T, B, nullptr, s)) return;
+            fusedForward<R>(v, X, B, nullptr, s);
+            fusedBackward<R>(v, T, B, s);
+        });
         // one chain per gradient up to kGradRows rows; above, chunks of rows
-        // fill the GPU (44 tiles of the tuner's network leave 108 SMs idle)
+        // fill the GPU (168 small tiles of the tuner's network fill it once, 42 large ones do not)
         const int rows = B <= kGradRows ? B : std::max(kGradChunk, ceilDiv(B, kGradChunks));
         const int chunks = ceilDiv(B, rows);
         const size_t stride = (numParams + 31) & ~(size_t)31;
         if (chunks > 1) part.ensure(stride * chunks);
-        kWeightGrad<<<dim3(tiles, chunks), 256, 0, s>>>(v, X, B, rows, grads.p, chunks > 1 ? part.p : nullptr, stride);
-        RACE_CUDA(cudaGetLastError());
+        if (chunks == 1) weightGrad<2, 1>(v, X, T, B, rows, chunks, stride, host, s);
+        else weightGrad<4, 2>(v, X, T, B, rows, chunks, stride, host, s);
         if (chunks > 1) {
             kGradReduce<<<ceilDiv((long long)numParams, 256), 256, 0, s>>>((long long)numParams, chunks, part.p, stride,
-                                                                          grads.p);
+                                                                          grads.p, host);
             RACE_CUDA(cudaGetLastError());
         }
     }
@@ -543,8 +828,8 @@ struct Mlp {
         return acts.p + actOff(layers(), B);
     }
     // loss and gradients of the MSE against targets T (B x out)
-    void lossGrad(const float *X, const float *T, int B, cudaStream_t s) {
-        if (fused) return lossGradFused(X, T, B, s);
+    void lossGrad(const float *X, const float *T, int B, float *host, cudaStream_t s) {
+        if (fused) return lossGradFused(X, T, B, host, s);
         float *y = forward(X, B, s);
         float *d = deltas.p, *dNext = deltas.p + deltas.n / 2;
         kMse<<<1, 256, 0, s>>>(B * out, y, T, d, loss());
@@ -651,15 +936,19 @@ int race_mlp_loss_grad(race_mlp *h, const float *X, const float *T, int batch, f
     if (!h || !X || !T || batch < 1) return RACE_ERR_INVALID_ARG;
     return guardMlp(h, [&] {
         cudaStream_t s = (cudaStream_t)stream;
-        h->net->lossGrad(X, T, batch, s);
-        if (!loss_host && !grad_host) return;
-        // one copy through pinned memory (a pageable copy waits by itself,
-        // and there were two)
+        // The kernels write what the caller wants to pinned memory themselves
+        // (52 -> 47 us a call of 239 rows); one product at a time copies it.
         race::Mlp &net = *h->net;
-        if (!net.hostGrads) RACE_CUDA(cudaMallocHost((void **)&net.hostGrads, sizeof(float) * (net.numParams + 1)));
-        const size_t first = grad_host ? 0 : net.numParams;
-        RACE_CUDA(cudaMemcpyAsync(net.hostGrads + first, net.grads.p + first, sizeof(float) * (net.numParams + 1 - first),
-                                  cudaMemcpyDeviceToHost, s));
+        const bool wanted = loss_host || grad_host;
+        if (wanted && !net.hostGrads)
+            RACE_CUDA(cudaMallocHost((void **)&net.hostGrads, sizeof(float) * (net.numParams + 1)));
+        net.lossGrad(X, T, batch, grad_host ? net.hostGrads : nullptr, s);
+        if (!wanted) return;
+        if (!net.fused || !grad_host) {
+            const size_t first = grad_host ? 0 : net.numParams;
+            RACE_CUDA(cudaMemcpyAsync(net.hostGrads + first, net.grads.p + first,
+                                      sizeof(float) * (net.numParams + 1 - first), cudaMemcpyDeviceToHost, s));
+        }
         RACE_CUDA(cudaStreamSynchronize(s));
         if (grad_host) std::memcpy(grad_host, net.hostGrads, sizeof(float) * net.numParams);
         if (loss_host) *loss_host = net.hostGrads[net.numParams];
