@@ -778,9 +778,17 @@ void buildFlow(Engine &e, FuncEntry &f, int dir, const FlowOrder &fo, const std:
 // One direction of a Gauss-Seidel or Kaczmarz function; leaf: the leaf
 // executor's sums, else the sequential ones.
 void runFlow(Engine &e, FuncEntry &f, int dir, bool leaf) {
-    if (f.ops.vec_type == RACE_VAL_F64) launchFlowK<double, double>(e, f, dir, leaf);
-    else if (f.ops.val_type == RACE_VAL_F32) launchFlowK<float, float>(e, f, dir, leaf);
-    else launchFlowK<__nv_bfloat16, float>(e, f, dir, leaf);
+    const race_operands &o = f.ops;
+    if (o.vec_type == RACE_VAL_F64) {
+        if (o.val_type != RACE_VAL_F64) throw Error(RACE_ERR_INVALID_ARG, "FP64 vectors need FP64 values");
+        launchFlowK<double, double>(e, f, dir, leaf);
+    } else if (o.vec_type == RACE_VAL_F32) {
+        if (o.val_type == RACE_VAL_F32) launchFlowK<float, float>(e, f, dir, leaf);
+        else if (o.val_type == RACE_VAL_BF16) launchFlowK<__nv_bfloat16, float>(e, f, dir, leaf);
+        else throw Error(RACE_ERR_INVALID_ARG, "FP32 vectors need FP32 or BF16 values");
+    } else {
+        throw Error(RACE_ERR_INVALID_ARG, "unknown vector type");
+    }
 }
 
 }  // namespace race
