@@ -573,19 +573,37 @@ __device__ __forceinline__ bool combTask(const FlowArgs &a, const int4 &t, int l
     return true;
 }
 
-// FLOW_SCAT: Kaczmarz update of a segment's entries with the row's scale.
+// FLOW_SCAT: Kaczmarz update of a segment's entries with the row's scale. The
+// segment's sum read the same words with their tags, but in another warp, and
+// relaxed accesses to the scale's word carry no order for these: the entries
+// are awaited again.
 template <typename VT, typename XT>
 __device__ __forceinline__ bool scatTask(const FlowArgs &a, const int4 &t, int lane) {
     const int idx[1] = {t.y}, want[1] = {1};
     XT sc[1];
     const bool ok = await<XT, 1>(a, a.segScl, idx, want, 1u, sc);
     if (__any_sync(0xffffffffu, !ok)) return false;
-    for (int j = t.z + lane; j < t.w; j += 32) {
-        const int c = a.col[j], m = a.mark[j];
-        XT xv;
-        int tag;
-        ldTag(a.xt, c, xv, tag);  // the segment's sum read it with its tag, and only this row may change it
-        kaczStore<XT>(a, c, m, mac(-sc[0], ld<VT, XT>((const VT *)a.val, j), xv));
+    constexpr int P = 4;
+    for (int j0 = t.z; j0 < t.w; j0 += 32 * P) {
+        XT v[P], xv[P];
+        int c[P], m[P];
+        unsigned valid = 0;
+#pragma unroll
+        for (int k = 0; k < P; ++k) {
+            const int j = j0 + 32 * k + lane;
+            v[k] = xv[k] = XT(0);
+            c[k] = m[k] = 0;
+            if (j < t.w) {
+                valid |= 1u << k;
+                v[k] = ld<VT, XT>((const VT *)a.val, j);
+                c[k] = a.col[j];
+                m[k] = a.mark[j];
+            }
+        }
+        if (__any_sync(0xffffffffu, !kaczValues<XT, P>(a, c, m, valid, xv))) return false;
+#pragma unroll
+        for (int k = 0; k < P; ++k)
+            if (valid >> k & 1) kaczStore<XT>(a, c[k], m[k], mac(-sc[0], v[k], xv[k]));
     }
     return true;
 }
