@@ -646,17 +646,17 @@ template <typename XT, bool KACZ>
 __global__ void __launch_bounds__(256) kFlowPrep(int n, int numSegs, const XT *__restrict__ x, void *xt,
                                                  XT *__restrict__ xold, void *segDot, void *segNrm, void *segScl,
                                                  int *status, int *ticket) {
-    const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
+    const long long i0 = blockIdx.x * blockDim.x + threadIdx.x;
     if (i0 == 0) {
         *status = DEV_OK;
         *ticket = 0;
     }
-    for (int i = i0; i < n; i += gridDim.x * blockDim.x) {
+    for (long long i = i0; i < n; i += gridDim.x * blockDim.x) {
         const XT v = x[i];
         if constexpr (!KACZ) xold[i] = v;
         stTag(xt, i, v, 0);
     }
-    for (int i = i0; i < numSegs; i += gridDim.x * blockDim.x) {
+    for (long long i = i0; i < numSegs; i += gridDim.x * blockDim.x) {
         stTag(segDot, i, XT(0), 0);
         if constexpr (KACZ) {
             stTag(segNrm, i, XT(0), 0);
@@ -668,7 +668,7 @@ __global__ void __launch_bounds__(256) kFlowPrep(int n, int numSegs, const XT *_
 // GS marks: a column whose row comes earlier in the order gets the sign bit.
 __global__ void kGsMarks(int n, const int *__restrict__ rowPtr, const int *__restrict__ col,
                          const int *__restrict__ order, int *__restrict__ mark) {
-    const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const long long r = warpOf(blockIdx.x, blockDim.x, threadIdx.x);
     if (r >= n) return;
     const int o = order[r];
     for (int j = rowPtr[r] + (threadIdx.x & 31); j < rowPtr[r + 1]; j += 32) {

@@ -12,6 +12,13 @@ namespace race {
 constexpr int kHugeRow = 512;
 constexpr int kHugeSeg = 256;
 
+// The warp that thread `thread` of block `block` belongs to, counted through
+// the grid. A warp per row needs 32 threads a row: beyond 2^27 rows their
+// number does not fit in 32 bits.
+__host__ __device__ constexpr long long warpOf(unsigned block, unsigned threadsPerBlock, unsigned thread) {
+    return ((long long)block * threadsPerBlock + thread) >> 5;
+}
+
 template <typename VT>
 __device__ __forceinline__ float toF(VT v) { return (float)v; }
 template <>
