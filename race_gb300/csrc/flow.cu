@@ -751,7 +751,7 @@ void buildFlow(Engine &e, FuncEntry &f, int dir, const FlowOrder &fo, const std:
                 const int cnt = std::min(32, p1 - p);
                 bool any = false;
                 for (int q = p; q < p + cnt; ++q) any |= len(q) <= mid;
-                if (any) seq.push_back(make_int4(FLOW_CHUNK, p, cnt, (int)waveChunk[wi] + (p - p0) / 32));
+                if (any) seq.push_back(make_int4(FLOW_CHUNK, p, cnt, waveChunk.at(wi) + (p - p0) / 32));
             }
         }
         // leaf arithmetic: four neighbouring rows of up to 32 products per

@@ -767,31 +767,29 @@ void buildSweepWaves(Engine &e, FuncEntry &f) {
         // into chunks of 32 positions whose width is their longest thread
         // row (SELL-C-sigma with sigma = the wave)
         const int mid = midRowOf(e, f);
-        std::vector<int> waveChunk{0}, cPos, cEnd, cLen;
+        std::vector<int> waveChunk{0}, cPos, cEnd, cLen;  // waveChunk: an entry per wave, with and without the copy
         std::vector<long long> cOff;
         long long slots = 0;
-        if (e.sweepSell) {
-            auto rowLen = [&](int r) { return rp[r + 1] - rp[r]; };
-            for (size_t wi = 0; wi < huge.size(); ++wi) {
-                if (!huge[wi]) {
-                    std::sort(rows.begin() + ptr[wi], rows.begin() + ptr[wi + 1], [&](int x, int y) {
-                        return rowLen(x) != rowLen(y) ? rowLen(x) > rowLen(y) : x < y;
-                    });
-                    for (int p0 = ptr[wi]; p0 < ptr[wi + 1]; p0 += 32) {
-                        const int p1 = std::min(p0 + 32, ptr[wi + 1]);
-                        int L = 0;
-                        for (int q = p0; q < p1; ++q)
-                            if (rowLen(rows[q]) <= mid) L = std::max(L, rowLen(rows[q]));
-                        L = (L + 3) & ~3;
-                        cPos.push_back(p0);
-                        cEnd.push_back(p1);
-                        cLen.push_back(L);
-                        cOff.push_back(slots);
-                        slots += 32LL * L;
-                    }
+        auto rowLen = [&](int r) { return rp[r + 1] - rp[r]; };
+        for (size_t wi = 0; wi < huge.size(); ++wi) {
+            if (e.sweepSell && !huge[wi]) {
+                std::sort(rows.begin() + ptr[wi], rows.begin() + ptr[wi + 1], [&](int x, int y) {
+                    return rowLen(x) != rowLen(y) ? rowLen(x) > rowLen(y) : x < y;
+                });
+                for (int p0 = ptr[wi]; p0 < ptr[wi + 1]; p0 += 32) {
+                    const int p1 = std::min(p0 + 32, ptr[wi + 1]);
+                    int L = 0;
+                    for (int q = p0; q < p1; ++q)
+                        if (rowLen(rows[q]) <= mid) L = std::max(L, rowLen(rows[q]));
+                    L = (L + 3) & ~3;
+                    cPos.push_back(p0);
+                    cEnd.push_back(p1);
+                    cLen.push_back(L);
+                    cOff.push_back(slots);
+                    slots += 32LL * L;
                 }
-                waveChunk.push_back((int)cPos.size());
             }
+            waveChunk.push_back((int)cPos.size());
         }
         w.numWaves = (int)huge.size();
         w.maxRows = 0;
