@@ -153,8 +153,8 @@ __device__ __forceinline__ void blockRows(const BlockMember &m, int r0, int r1, 
     }
 }
 
-// Relaxed polls and one acquire fence after the successful one (an acquire
-// load per flag empties the L1 each time).
+// Relaxed polls, one acquire fence after the successful one (an acquire load
+// per flag empties the L1 each time) and a warp barrier behind the fence.
 template <typename VT, typename XT, int R>
 __global__ void __launch_bounds__(kBlockThreads) kMpkBlock(BlockArgs a) {
     const int lane = threadIdx.x & 31;
@@ -182,6 +182,7 @@ __global__ void __launch_bounds__(kBlockThreads) kMpkBlock(BlockArgs a) {
                 __nanosleep(32);
             }
             asm volatile("fence.acq_rel.gpu;" ::: "memory");
+            __syncwarp();  // a lane reads what other lanes' flags stand for; the vote orders nothing
         }
         for (int r = h.x; r < h.y; r += 32) blockRows<VT, XT, R>(m, r, min(h.y, r + 32), k);
         __syncwarp();

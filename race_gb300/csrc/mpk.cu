@@ -427,7 +427,8 @@ struct MpkArgs {
 // warps, so the wait always ends (bounded anyway: a timeout goes to the
 // status word). The polls are relaxed loads and one acquire fence follows
 // the successful poll (a counter read by a relaxed load and a later
-// fence.acq_rel form an acquire of the writers' releases). A warp takes the
+// fence.acq_rel form an acquire of the writers' releases), then a warp
+// barrier, since each lane polled other counters. A warp takes the
 // runs of its own die's queue, so each chunk's matrix block is cached by
 // one die's L2 only; an empty queue sends it to the other one. A warp adds
 // its previous run's chunks to their block counters (release reductions)
@@ -496,6 +497,7 @@ __global__ void __launch_bounds__(kWarpThreads, kMpkMinBlocks) kMpk(MpkArgs a) {
                 __nanosleep(32);
             }
             asm volatile("fence.acq_rel.gpu;" ::: "memory");
+            __syncwarp();  // a lane reads what other lanes' counters stand for; the vote orders nothing
         }
         const unsigned long long pol = (h.w & 1) ? polDrop : polKeep;
         for (int c = h.x; c < h.y; ++c) chunkRow<VT, HUBS, C16, true>(a.m, c, k, a.n, a.x, a.xf, pol);
@@ -588,6 +590,7 @@ __device__ __forceinline__ void hubTask(const SellView &m, const HubWork &hw, in
             }
             if (!__shfl_sync(0xffffffffu, last, 0)) return;
             __threadfence();
+            __syncwarp();  // every lane behind the fence of lane 0, which read the counter
             t = AT(0);
             for (int g = lane; g < segs; g += 32) t += __ldcg(part + first + g);
 #pragma unroll

@@ -183,6 +183,7 @@ __global__ void __launch_bounds__(kNaThreads) kMpkNoAlloc(NaArgs a) {
                 }
                 __nanosleep(32);
             }
+            __syncwarp();  // a lane reads what other lanes' flags stand for; the vote orders nothing
         }
         const double *xin = a.x + (size_t)k * a.n;
         if (live && e - s <= kMpkHubRowLen) {
