@@ -692,8 +692,17 @@ struct Mlp {
         }
         acts.alloc(total);
         deltas.alloc(fused ? total : 2 * widest);
+        if (fused && gradChunks(B) > 1) part.ensure(gradStride() * gradChunks(B));
         batchCap = B;
     }
+    // Rows that one chain of the fused weight gradients sums, and their chunks:
+    // one chain per gradient up to kGradRows rows; above, chunks of rows fill
+    // the GPU (168 small tiles of the tuner's network fill it once, 42 large
+    // ones do not). More rows never mean fewer chunks, so the workspace of a
+    // batch serves every smaller one.
+    static int gradRows(int B) { return B <= kGradRows ? B : std::max(kGradChunk, ceilDiv(B, kGradChunks)); }
+    static int gradChunks(int B) { return ceilDiv(B, gradRows(B)); }
+    size_t gradStride() const { return (numParams + 31) & ~(size_t)31; }
     NetView view(int B) const {
         NetView v{};
         v.layers = layers();
@@ -761,6 +770,11 @@ struct Mlp {
         }
         RACE_CUDA(cudaGetLastError());
     }
+    static bool capturing(cudaStream_t s) {
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        RACE_CUDA(cudaStreamIsCapturing(s, &st));
+        return st != cudaStreamCaptureStatusNone;
+    }
     // outputs only, to Y
     void predict(const float *X, int B, float *Y, cudaStream_t s) {
         if (!fused) {
@@ -768,6 +782,9 @@ struct Mlp {
             RACE_CUDA(cudaMemcpyAsync(Y, y, sizeof(float) * B * out, cudaMemcpyDeviceToDevice, s));
             return;
         }
+        // Outputs alone need no workspace, but the first pass of a batch size
+        // is also a later captured training pass's chance to allocate.
+        if (B > batchCap && !capturing(s)) ensure(B);
         const NetView v = view(0);
         byRows(B, [&](auto r) {
             constexpr int R = decltype(r)::value;
@@ -800,12 +817,8 @@ struct Mlp {
             fusedForward<R>(v, X, B, nullptr, s);
             fusedBackward<R>(v, T, B, s);
         });
-        // one chain per gradient up to kGradRows rows; above, chunks of rows
-        // fill the GPU (168 small tiles of the tuner's network fill it once, 42 large ones do not)
-        const int rows = B <= kGradRows ? B : std::max(kGradChunk, ceilDiv(B, kGradChunks));
-        const int chunks = ceilDiv(B, rows);
-        const size_t stride = (numParams + 31) & ~(size_t)31;
-        if (chunks > 1) part.ensure(stride * chunks);
+        const int rows = gradRows(B), chunks = gradChunks(B);
+        const size_t stride = gradStride();
         if (chunks == 1) weightGrad<2, 1>(v, X, T, B, rows, chunks, stride, host, s);
         else weightGrad<4, 2>(v, X, T, B, rows, chunks, stride, host, s);
         if (chunks > 1) {
