@@ -785,11 +785,17 @@ struct Mlp {
         // Outputs alone need no workspace, but the first pass of a batch size
         // is also a later captured training pass's chance to allocate.
         if (B > batchCap && !capturing(s)) ensure(B);
+        // Blocks write outputs while others still read inputs: outputs that
+        // share memory with the inputs are put together apart from them.
+        const bool overlap = Y < X + (size_t)B * in && X < Y + (size_t)B * out;
+        if (overlap) ensure(B);
+        float *y = overlap ? acts.p + actOff(layers(), B) : Y;
         const NetView v = view(0);
         byRows(B, [&](auto r) {
             constexpr int R = decltype(r)::value;
-            if (!residentPass<R, false>(v, X, nullptr, B, Y, s)) fusedForward<R>(v, X, B, Y, s);
+            if (!residentPass<R, false>(v, X, nullptr, B, y, s)) fusedForward<R>(v, X, B, y, s);
         });
+        if (overlap) RACE_CUDA(cudaMemcpyAsync(Y, y, sizeof(float) * B * out, cudaMemcpyDeviceToDevice, s));
     }
     template <int NW, int KW>
     void weightGrad(const NetView &v, const float *X, const float *T, int B, int rows, int chunks, size_t stride,
