@@ -683,6 +683,11 @@ struct Mlp {
         for (int i = 1; i < l; ++i) o += (size_t)B * dimOut[i - 1];
         return o;
     }
+    // A batch is limited by the second grid dimension of kGemm; the fused
+    // passes count rows and outputs in 32 bits within it.
+    static void checkBatch(int B) {
+        if (B > 65535 * kT) throw Error(RACE_ERR_INVALID_ARG, "a batch holds at most 2,097,120 rows");
+    }
     void ensure(int B) {
         if (B <= batchCap) return;
         size_t total = 0, widest = 0;
@@ -946,6 +951,7 @@ int race_mlp_get_params(race_mlp *h, float *host, long long count) {
 int race_mlp_forward(race_mlp *h, const float *X, int batch, float *Y, void *stream) {
     if (!h || !X || !Y || batch < 1) return RACE_ERR_INVALID_ARG;
     return guardMlp(h, [&] {
+        race::Mlp::checkBatch(batch);
         h->net->predict(X, batch, Y, (cudaStream_t)stream);
     });
 }
@@ -958,6 +964,7 @@ int race_mlp_loss_grad(race_mlp *h, const float *X, const float *T, int batch, f
         // The kernels write what the caller wants to pinned memory themselves
         // (52 -> 47 us a call of 239 rows); one product at a time copies it.
         race::Mlp &net = *h->net;
+        race::Mlp::checkBatch(batch);
         const bool wanted = loss_host || grad_host;
         if (wanted && !net.hostGrads)
             RACE_CUDA(cudaMallocHost((void **)&net.hostGrads, sizeof(float) * (net.numParams + 1)));
