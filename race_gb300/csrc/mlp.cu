@@ -648,6 +648,7 @@ struct Mlp {
     DevBuf<float> part;          // gradients of chunks of rows
     float *hostGrads = nullptr;  // pinned: gradients and loss on their way to the caller
     bool fused = false;          // one kernel per pass (else one per product)
+    unsigned sharedAllowed = 0;  // allowShared's kernels, a bit each
     int batchCap = 0;
     long long steps = 0;
 
@@ -732,18 +733,23 @@ struct Mlp {
     // blocks, 18.5 us for loss and gradients, 4 rows 20.5), then 4 and 8, and 16
     // where enough blocks remain to share each weight among more rows.
     static int rowsPerBlock(int B) { return B <= 2 * 152 ? 2 : B <= 4 * 152 ? 4 : B <= 8 * 152 ? 8 : 16; }
+    // Lets a kernel take more than 48 KB of shared memory. That holds for one
+    // device, the network's own, so each network asks once per kernel (slot).
+    static int rowsIndex(int R) { return R == 2 ? 0 : R == 4 ? 1 : R == 8 ? 2 : 3; }
+    template <typename K>
+    void allowShared(K kernel, int slot, int bytes) {
+        if (sharedAllowed >> slot & 1) return;
+        RACE_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+        sharedAllowed |= 1u << slot;
+    }
     template <int R>
     void fusedForward(const NetView &v, const float *X, int B, float *y, cudaStream_t s) {
-        static const cudaError_t opt = cudaFuncSetAttribute(
-            kForward<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, passBytes(R, kFusedDim));
-        RACE_CUDA(opt);
+        allowShared(kForward<R>, 0 + rowsIndex(R), passBytes(R, kFusedDim));
         kForward<R><<<ceilDiv(B, R), 256, passBytes(R, rowStride()), s>>>(v, X, B, rowStride(), y);
     }
     template <int R>
     void fusedBackward(const NetView &v, const float *T, int B, cudaStream_t s) {
-        static const cudaError_t opt = cudaFuncSetAttribute(
-            kBackward<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, passBytes(R, kFusedDim));
-        RACE_CUDA(opt);
+        allowShared(kBackward<R>, 4 + rowsIndex(R), passBytes(R, kFusedDim));
         kBackward<R><<<ceilDiv(B, R), 256, passBytes(R, rowStride()), s>>>(v, T, B, rowStride());
     }
     // Shared memory of the whole network and R rows of two layers (164 KB for
@@ -758,9 +764,7 @@ struct Mlp {
     bool residentPass(const NetView &v, const float *X, const float *T, int B, float *y, cudaStream_t s) {
         const size_t bytes = residentBytes(R);
         if (bytes > kResidentBytes) return false;
-        static const cudaError_t opt = cudaFuncSetAttribute(
-            kResident<R, TRAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kResidentBytes);
-        RACE_CUDA(opt);
+        allowShared(kResident<R, TRAIN>, (TRAIN ? 12 : 8) + rowsIndex(R), (int)kResidentBytes);
         const int perSm = (int)std::max<size_t>(1, std::min<size_t>(8, kResidentBytes / (bytes + 1024)));
         kResident<R, TRAIN><<<std::min(ceilDiv(B, R), kResidentSms * perSm), 256, bytes, s>>>(v, X, T, B, rowStride(), y);
         return true;
