@@ -1329,6 +1329,29 @@ void launchSpmvSell(const MpkPlan &p, int n, int k, double *x, cudaStream_t s) {
         else launchSpmvSellK<VT, false, false>(p, n, k, x, s);
     }
 }
+
+// Loads the code of both schedules' kernels, which CUDA otherwise does at
+// their first launch.
+template <typename VT, bool HUBS, bool C16>
+void loadSchedulesK(const MpkPlan &p) {
+    cudaFuncAttributes fa;
+    RACE_CUDA(cudaFuncGetAttributes(&fa, kMpk<VT, HUBS, C16>));
+    if (HUBS || p.numChunks <= kSmallWarpsPerSm * devSms())
+        RACE_CUDA(cudaFuncGetAttributes(&fa, kSpmvSellSmall<VT, HUBS, C16>));
+    else
+        RACE_CUDA(cudaFuncGetAttributes(&fa, kSpmvSell<VT, C16>));
+}
+
+template <typename VT>
+void loadSchedules(const MpkPlan &p) {
+    if (p.numHubs > 0) {
+        if (p.col16) loadSchedulesK<VT, true, true>(p);
+        else loadSchedulesK<VT, true, false>(p);
+    } else {
+        if (p.col16) loadSchedulesK<VT, false, true>(p);
+        else loadSchedulesK<VT, false, false>(p);
+    }
+}
 }  // namespace
 
 namespace {
@@ -1375,15 +1398,25 @@ void runSweeps(MpkPlan &plan, const race_operands &ops, cudaStream_t s) {
 }
 
 // RACE_MPK_AUTO's choice: each schedule timed on its second run (the first
-// warms the code and the caches), the faster kept; a first run more than
-// twice as slow as the other's settles it (a small matrix's or a hub-row
-// matrix's wavefront is 4 to 25 times slower). Both compute the same powers,
-// so the call's result is complete either way; the wavefront's status word is
-// cleared afterwards, as the sweeps would leave it.
+// warms the caches), the faster kept; a first run more than twice as slow as
+// the other's settles it (a small matrix's or a hub-row matrix's wavefront is
+// 4 to 25 times slower). The code of both is loaded before, so that a first
+// run does not depend on what the process ran earlier: loading a kernel
+// between the events took 15 to 30 us (7-point 24^3, FP32: plain launches 29
+// us in their first run with loading, 15 us without, 12 us in the second; the
+// wavefront 68, 57 and 54 us). Both compute the same powers, so the call's
+// result is complete either way; the wavefront's status word is cleared
+// afterwards, as the sweeps would leave it.
 int chooseSchedule(MpkPlan &plan, const race_operands &ops, cudaStream_t s) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     RACE_CUDA(cudaStreamIsCapturing(s, &cs));
     if (cs != cudaStreamCaptureStatusNone) return plan.valType == RACE_VAL_F64 ? RACE_MPK_WAVEFRONT : RACE_MPK_SWEEPS;
+    switch (plan.valType) {
+    case RACE_VAL_F64: loadSchedules<double>(plan); break;
+    case RACE_VAL_F32: loadSchedules<float>(plan); break;
+    case RACE_VAL_BF16: loadSchedules<__nv_bfloat16>(plan); break;
+    default: throw Error(RACE_ERR_INVALID_ARG, "unknown value type");
+    }
     cudaEvent_t ev[2];
     RACE_CUDA(cudaEventCreate(&ev[0]));
     RACE_CUDA(cudaEventCreate(&ev[1]));
