@@ -235,6 +235,8 @@ class Engine {
     // order (coalesced vector loads) instead of the caller's CRS.
     int sweepMidRow = -1;
     bool sweepSell = true;
+    // dataflow sweeps: polls after which a wait gives up (in steps of 64)
+    long long sweepMaxPolls = kSpinLimit;
 
     // coloring results
     std::unique_ptr<ZoneTree> tree;

@@ -120,16 +120,18 @@ struct FlowArgs {
     const long long *chunkOff;  // SELL copy of the short rows (sellCol: GS marks), or null
     const void *sellVal;
     const int *sellCol, *sellMark;
+    long long maxPolls;  // of one wait
     int *status, *ticket;
 };
 
-// The spin limit of a wait: false once it is passed, or another warp has
-// reported one (the status word is then set).
+// The limit of a wait: false once it is passed, or another warp has reported
+// one (the status word is then set). The lanes' answers are joined: a lane
+// that saw the word before it was set would wait for the others otherwise.
 __device__ __forceinline__ bool mayWait(const FlowArgs &a, long long &spins) {
     if ((++spins & 63) != 0) return true;
     int st;
     asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(st) : "l"(a.status) : "memory");
-    if (spins <= kSpinLimit && st == DEV_OK) return true;
+    if (!__any_sync(0xffffffffu, spins > a.maxPolls || st != DEV_OK)) return true;
     atomicCAS(a.status, DEV_OK, DEV_WAIT_TIMEOUT);
     return false;
 }
@@ -152,7 +154,7 @@ __device__ __forceinline__ bool await(const FlowArgs &a, const void *words, cons
         for (int k = 0; k < N; ++k)
             if ((todo >> k & 1) && tag[k] == want[k]) todo &= ~(1u << k);
         if (!__any_sync(0xffffffffu, todo != 0)) return true;
-        if (!mayWait(a, spins)) return false;  // the same count in every lane
+        if (!mayWait(a, spins)) return false;  // the whole warp
     }
 }
 
@@ -703,7 +705,7 @@ void launchFlow(Engine &e, FuncEntry &f, int dir, bool leaf) {
     RACE_CUDA(cudaGetLastError());
     FlowArgs a{o.col, o.val, o.x, o.b, w.task[leaf].p, T, w.pos.p, w.mark.p, f.flowX.p, f.flowOld.p,
                seg, seg + word * S, seg + 2 * word * S, wv.sellMidRow,
-               wv.sell ? wv.chunkOff.p : nullptr, wv.sellVal.p, wv.sellCol.p, w.sellMark.p, status, ticket};
+               wv.sell ? wv.chunkOff.p : nullptr, wv.sellVal.p, wv.sellCol.p, w.sellMark.p, e.sweepMaxPolls, status, ticket};
     void *args[] = {&a};
     const int blocks = std::max(1, std::min(resident, ceilDiv(T, kFlowWarps)));
     RACE_CUDA(cudaLaunchCooperativeKernel((void *)kFlow<VT, XT, KACZ>, blocks, kFlowThreads, args, 0, e.stream));

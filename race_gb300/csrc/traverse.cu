@@ -291,6 +291,7 @@ Engine::Engine(int nrow, int nthreads, int dist_, const int *rowPtr, const int *
     if (const char *c16 = getenv("RACE_GPU_MPK_COL16")) mpkCol16 = atoi(c16) != 0;
     if (const char *mr = getenv("RACE_GPU_SWEEP_MIDROW")) sweepMidRow = std::max(-1, atoi(mr));
     if (const char *ss = getenv("RACE_GPU_SWEEP_SELL")) sweepSell = atoi(ss) != 0;
+    if (const char *mp = getenv("RACE_GPU_SWEEP_MAX_POLLS")) sweepMaxPolls = std::max(0LL, atoll(mp));
     if (const char *sc = getenv("RACE_GPU_MPK_SCHEDULE"))
         mpkSchedule = std::string(sc) == "wavefront" ? RACE_MPK_WAVEFRONT
                       : std::string(sc) == "sweeps"  ? RACE_MPK_SWEEPS
