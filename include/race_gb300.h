@@ -158,9 +158,11 @@ int race_register_function(race_engine *e, int kernel, const race_operands *ops,
  * RACE_ERR_TIMEOUT if a device wait gave up. */
 int race_execute_function(race_engine *e, int func_id, int rev);
 /* Same work without waiting (stream-ordered, like a CUDA library call);
- * race_get_status later synchronises and reports the device status word of
- * the last launch. No counterpart in the reference, whose executor is
- * synchronous. */
+ * race_get_status later synchronises and returns RACE_ERR_TIMEOUT, once, if
+ * a device wait of any launch since the last report gave up (a synchronous
+ * call reports earlier ones too). Gauss-Seidel and Kaczmarz sweeps enqueued
+ * behind one that gave up do nothing until then. No counterpart in the
+ * reference, whose executor is synchronous. */
 int race_execute_function_async(race_engine *e, int func_id, int rev);
 int race_get_status(race_engine *e);
 /* RACE_SWEEP_GATHER runs SpMV, SpMTV and SymmSpMV without the coloring's
@@ -293,8 +295,8 @@ int race_register_mpk_block(race_engine *e, const race_operands *ops, int power,
  * graph and replays the graph on every call (inputs are read through the
  * recorded pointers, so new data in the same buffers is picked up).
  * race_batch_get_status synchronises `stream` and returns RACE_ERR_TIMEOUT
- * if a device wait of the last launch gave up. race_batch_info reports
- * members, chunks and work items (0 before prepare). */
+ * (once) if a device wait of a launch since the last report gave up.
+ * race_batch_info reports members, chunks and work items (0 before prepare). */
 typedef struct race_batch race_batch;
 int race_batch_create(race_batch **out);
 int race_batch_destroy(race_batch *b);

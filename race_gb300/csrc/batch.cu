@@ -394,12 +394,11 @@ std::unique_ptr<BlockPlan> buildBlockPlan(Engine &e, const race_operands &ops, i
 
 // Resets the completion flags, ticket and status word and launches the
 // persistent kernel: all stream-ordered, so the sequence can be captured.
-void runBatch(BatchTables &t, cudaStream_t s) {
+void runBatch(BatchTables &t, int *status, cudaStream_t s) {
     RACE_CUDA(cudaMemsetAsync(t.done.p, 0, sizeof(int) * (size_t)t.maxPower * t.numChunks, s));
     RACE_CUDA(cudaMemsetAsync(t.ticket.p, 0, sizeof(int), s));
-    RACE_CUDA(cudaMemsetAsync(t.status.p, 0, sizeof(int), s));
     if (t.numItems == 0) return;
-    BlockArgs a{t.members.p, t.item.p, t.numItems, t.numChunks, t.done.p, t.ticket.p, t.status.p};
+    BlockArgs a{t.members.p, t.item.p, t.numItems, t.numChunks, t.done.p, t.ticket.p, status};
     dispatch<LaunchBlockFn>(t.valType, t.vecType, t.nrhs, a, s);
     RACE_CUDA(cudaGetLastError());
 }

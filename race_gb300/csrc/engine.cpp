@@ -26,7 +26,7 @@ void symmGsIr(Engine &e, int inner, int n, const int *rowPtr, const int *col, co
               double *x, double tol, int maxIter, int sweeps, int *itersOut, double *relresOut);
 std::unique_ptr<BlockPlan> buildBlockPlan(Engine &e, const race_operands &ops, int power, int nrhs);
 void buildBatchTables(BatchTables &t, const std::vector<const BlockPlan *> &plans, cudaStream_t s);
-void runBatch(BatchTables &t, cudaStream_t s);
+void runBatch(BatchTables &t, int *status, cudaStream_t s);
 void runBlockSpmv(const BlockPlan &p, int k, cudaStream_t s);
 
 // Interface::RACEColor() (interface.cpp:260-301): level recursion over the
@@ -200,20 +200,32 @@ void Engine::launch(int id, bool rev) {
     if (id < 0 || id >= (int)funcs.size()) throw Error(RACE_ERR_INVALID_ARG, "unknown function id");
     FuncEntry &f = funcs[id];
     if (f.block) {
-        runBatch(f.block->tables, stream);
-        lastStatus = f.block->tables.status.p;
+        noteWaits();
+        runBatch(f.block->tables, dStatus.p, stream);
     } else if (f.kernel == RACE_K_MPK) {
-        runMpk(*this, *f.mpk, f.ops, f.power);  // sets lastStatus
+        runMpk(*this, *f.mpk, f.ops, f.power);
     } else {
-        runSweep(*this, f, rev);  // sets lastStatus
+        runSweep(*this, f, rev);
     }
 }
 
+void Engine::noteWaits() {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    RACE_CUDA(cudaStreamIsCapturing(stream, &cs));
+    (cs == cudaStreamCaptureStatusNone ? waitsUnread : waitsCaptured) = true;
+}
+
+// Reports the launches since the last report, each failure once.
 void Engine::checkStatus() {
-    int st = 0;
-    if (lastStatus) RACE_CUDA(cudaMemcpyAsync(&st, lastStatus, sizeof(int), cudaMemcpyDeviceToHost, stream));
+    int st = DEV_OK;
+    if (waitsUnread || waitsCaptured)
+        RACE_CUDA(cudaMemcpyAsync(&st, dStatus.p, sizeof(int), cudaMemcpyDeviceToHost, stream));
     RACE_CUDA(cudaStreamSynchronize(stream));
-    if (st != DEV_OK) throw Error(RACE_ERR_TIMEOUT, "a device wait gave up (schedule dependency or grid barrier)");
+    waitsUnread = false;
+    if (st == DEV_OK) return;
+    RACE_CUDA(cudaMemsetAsync(dStatus.p, 0, sizeof(int), stream));
+    RACE_CUDA(cudaStreamSynchronize(stream));
+    throw Error(RACE_ERR_TIMEOUT, "a device wait gave up (schedule dependency or grid barrier)");
 }
 
 void Engine::execute(int id, bool rev) {
@@ -997,7 +1009,7 @@ int race_batch_execute(race_batch *b, void *stream) {
     if (!b) return RACE_ERR_INVALID_ARG;
     return guardBatch(b, [&] {
         if (!b->prepared) b->prepare((cudaStream_t)stream);
-        race::runBatch(b->tables, (cudaStream_t)stream);
+        race::runBatch(b->tables, b->tables.status.p, (cudaStream_t)stream);
     });
 }
 
@@ -1009,7 +1021,7 @@ int race_batch_graph_launch(race_batch *b, void *stream) {
             if (!b->capture) RACE_CUDA(cudaStreamCreateWithFlags(&b->capture, cudaStreamNonBlocking));
             RACE_CUDA(cudaStreamBeginCapture(b->capture, cudaStreamCaptureModeRelaxed));
             try {
-                race::runBatch(b->tables, b->capture);
+                race::runBatch(b->tables, b->tables.status.p, b->capture);
             } catch (...) {
                 cudaGraph_t g = nullptr;
                 cudaStreamEndCapture(b->capture, &g);
@@ -1030,7 +1042,10 @@ int race_batch_get_status(race_batch *b, void *stream) {
         int st = 0;
         RACE_CUDA(cudaMemcpyAsync(&st, b->tables.status.p, sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
         RACE_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
-        if (st != race::DEV_OK) throw Error(RACE_ERR_TIMEOUT, "a device wait gave up (schedule dependency)");
+        if (st == race::DEV_OK) return;
+        RACE_CUDA(cudaMemsetAsync(b->tables.status.p, 0, sizeof(int), (cudaStream_t)stream));
+        RACE_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
+        throw Error(RACE_ERR_TIMEOUT, "a device wait gave up (schedule dependency)");
     });
 }
 

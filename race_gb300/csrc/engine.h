@@ -78,7 +78,7 @@ struct MpkPlan {
     DevBuf<int> blockStart;     // numBlocks+1
     DevBuf<int> done;           // power * numBlocks: chunks complete per block
     DevBuf<int> ticket;         // next run of each die queue
-    DevBuf<int> status;         // 1: device status word
+    DevBuf<int> status;         // 1: status word of the timed runs (chooseSchedule)
     // Triangular partitions (mtxType L/U): a row may read any earlier group,
     // so the items run as one launch per wavefront step, without waits;
     // items stepPtr[s] .. stepPtr[s+1]) form step s.
@@ -181,9 +181,9 @@ struct FuncEntry {
     DevWaves waves[2];  // forward, reverse
     DevFlow flow[2];
     // dataflow executor, both directions: (value, tag) copy of x, x before
-    // the sweep, status word and ticket
+    // the sweep, and the ticket
     DevBuf<unsigned char> flowX, flowOld;
-    DevBuf<int> flowCtl;
+    DevBuf<int> flowTicket;
     DevGather gather[2];
 };
 
@@ -205,7 +205,10 @@ class Engine {
     void execute(int id, bool rev);
     void launch(int id, bool rev);
     void checkStatus();
-    int *lastStatus = nullptr;  // device status word of the last launch
+    // A launch with bounded waits has been enqueued: the status word has to be
+    // read, and again and again if the launch was captured for replays.
+    void noteWaits();
+    bool waitsUnread = false, waitsCaptured = false;
     void spmvPlain(int n, const int *rowPtr, const int *col, const double *val, const double *x, double *b);
 
     int n = 0;
@@ -286,6 +289,9 @@ class Engine {
     LevelData powerLevels;
 
     std::vector<FuncEntry> funcs;
+    // [0]: status word of the engine's launches. A wait that gives up sets it,
+    // no launch clears it, checkStatus does once it has reported it. [2], [3]:
+    // counters of the grid barrier, cleared by each launch that has one.
     DevBuf<int> dStatus;
 };
 

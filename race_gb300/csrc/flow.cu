@@ -615,11 +615,16 @@ __global__ void __launch_bounds__(kFlowThreads, 1) kFlow(FlowArgs a) {
     __shared__ FlowStage<XT> stage;
     const int lane = threadIdx.x & 31;
     const int nw = gridDim.x * kFlowWarps;
+    // behind a sweep that gave up and has not been reported yet nothing runs
+    // (read along with the first task: no round trip of its own)
+    int st;
+    asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(st) : "l"(a.status) : "memory");
     int it = (blockIdx.x * kFlowThreads + threadIdx.x) >> 5;
     while (it < a.numTasks) {
         int next = 0;
         if (lane == 0) next = nw + atomicAdd(a.ticket, 1);  // the round trip overlaps this task
         const int4 t = a.task[it];
+        if (__any_sync(0xffffffffu, st != DEV_OK)) return;
         bool ok = true;
         switch (t.x) {
         case FLOW_CHUNK: ok = chunkTask<VT, XT, KACZ>(a, t, lane); break;
@@ -643,16 +648,13 @@ __global__ void __launch_bounds__(kFlowThreads, 1) kFlow(FlowArgs a) {
 }
 
 // Start of a sweep: the (value, tag) copy of x with tags 0, the old x of a
-// Gauss-Seidel sweep, the segments' tags, the status word and the ticket.
+// Gauss-Seidel sweep, the segments' tags and the ticket.
 template <typename XT, bool KACZ>
 __global__ void __launch_bounds__(256) kFlowPrep(int n, int numSegs, const XT *__restrict__ x, void *xt,
                                                  XT *__restrict__ xold, void *segDot, void *segNrm, void *segScl,
-                                                 int *status, int *ticket) {
+                                                 int *ticket) {
     const long long i0 = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i0 == 0) {
-        *status = DEV_OK;
-        *ticket = 0;
-    }
+    if (i0 == 0) *ticket = 0;
     for (long long i = i0; i < n; i += gridDim.x * blockDim.x) {
         const XT v = x[i];
         if constexpr (!KACZ) xold[i] = v;
@@ -694,18 +696,15 @@ void launchFlow(Engine &e, FuncEntry &f, int dir, bool leaf) {
     const int n = o.n, S = wv.numSegs, T = w.numTasks[leaf];
     constexpr size_t word = TagWord<XT>::kBytes;
     char *seg = (char *)w.segWords.p;
-    int *status = f.flowCtl.p, *ticket = f.flowCtl.p + 1;
-    if (T == 0) {
-        RACE_CUDA(cudaMemsetAsync(status, 0, sizeof(int), e.stream));
-        return;
-    }
+    int *ticket = f.flowTicket.p;
+    if (T == 0) return;
     const int prepBlocks = std::min(ceilDiv(std::max(n, S), 256), 152 * 8);
     kFlowPrep<XT, KACZ><<<prepBlocks, 256, 0, e.stream>>>(n, S, (const XT *)o.x, f.flowX.p, (XT *)f.flowOld.p, seg,
-                                                          seg + word * S, seg + 2 * word * S, status, ticket);
+                                                          seg + word * S, seg + 2 * word * S, ticket);
     RACE_CUDA(cudaGetLastError());
     FlowArgs a{o.col, o.val, o.x, o.b, w.task[leaf].p, T, w.pos.p, w.mark.p, f.flowX.p, f.flowOld.p,
                seg, seg + word * S, seg + 2 * word * S, wv.sellMidRow,
-               wv.sell ? wv.chunkOff.p : nullptr, wv.sellVal.p, wv.sellCol.p, w.sellMark.p, e.sweepMaxPolls, status, ticket};
+               wv.sell ? wv.chunkOff.p : nullptr, wv.sellVal.p, wv.sellCol.p, w.sellMark.p, e.sweepMaxPolls, e.dStatus.p, ticket};
     void *args[] = {&a};
     const int blocks = std::max(1, std::min(resident, ceilDiv(T, kFlowWarps)));
     RACE_CUDA(cudaLaunchCooperativeKernel((void *)kFlow<VT, XT, KACZ>, blocks, kFlowThreads, args, 0, e.stream));
@@ -780,7 +779,7 @@ void buildFlow(Engine &e, FuncEntry &f, int dir, const FlowOrder &fo, const std:
     w.segWords.alloc(std::max<size_t>(3 * word * segBeg.size(), 16));
     f.flowX.ensure(std::max<size_t>(word * n, 16));
     if (!kacz) f.flowOld.ensure(std::max<size_t>(word / 2 * n, 16));
-    f.flowCtl.ensure(2);
+    f.flowTicket.ensure(1);
     const size_t nnz = std::max(rp[n], 1);
     if (kacz) {
         w.mark.upload(fo.mark.empty() ? nullptr : fo.mark.data(), nnz, s);

@@ -1356,8 +1356,7 @@ void loadSchedules(const MpkPlan &p) {
 
 namespace {
 // The persistent wavefront kernel over all powers.
-void runWavefront(MpkPlan &plan, const race_operands &ops, cudaStream_t s) {
-    RACE_CUDA(cudaMemsetAsync(plan.status.p, 0, sizeof(int), s));
+void runWavefront(MpkPlan &plan, const race_operands &ops, int *status, cudaStream_t s) {
     RACE_CUDA(cudaMemsetAsync(plan.done.p, 0, sizeof(int) * (size_t)plan.numBlocks * plan.power, s));
     RACE_CUDA(cudaMemsetAsync(plan.ticket.p, 0, sizeof(int) * 2, s));
     MpkArgs a{viewOf(plan),
@@ -1370,7 +1369,7 @@ void runWavefront(MpkPlan &plan, const race_operands &ops, cudaStream_t s) {
               plan.blockStart.p,
               plan.done.p,
               plan.ticket.p,
-              plan.status.p,
+              status,
               plan.hints,
               plan.smDie,
               plan.numDies,
@@ -1405,8 +1404,8 @@ void runSweeps(MpkPlan &plan, const race_operands &ops, cudaStream_t s) {
 // between the events took 15 to 30 us (7-point 24^3, FP32: plain launches 29
 // us in their first run with loading, 15 us without, 12 us in the second; the
 // wavefront 68, 57 and 54 us). Both compute the same powers, so the call's
-// result is complete either way; the wavefront's status word is cleared
-// afterwards, as the sweeps would leave it.
+// result is complete either way; a wait that gives up here (in a status word of
+// the plan's own) only decides for the sweeps.
 int chooseSchedule(MpkPlan &plan, const race_operands &ops, cudaStream_t s) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     RACE_CUDA(cudaStreamIsCapturing(s, &cs));
@@ -1417,6 +1416,7 @@ int chooseSchedule(MpkPlan &plan, const race_operands &ops, cudaStream_t s) {
     case RACE_VAL_BF16: loadSchedules<__nv_bfloat16>(plan); break;
     default: throw Error(RACE_ERR_INVALID_ARG, "unknown value type");
     }
+    RACE_CUDA(cudaMemsetAsync(plan.status.p, 0, sizeof(int), s));
     cudaEvent_t ev[2];
     RACE_CUDA(cudaEventCreate(&ev[0]));
     RACE_CUDA(cudaEventCreate(&ev[1]));
@@ -1425,7 +1425,7 @@ int chooseSchedule(MpkPlan &plan, const race_operands &ops, cudaStream_t s) {
         if (rep == 1 && (ms[0] > 2 * ms[1] || ms[1] > 2 * ms[0])) break;
         for (int sc = 0; sc < 2; ++sc) {
             RACE_CUDA(cudaEventRecord(ev[0], s));
-            if (sc == 0) runWavefront(plan, ops, s);
+            if (sc == 0) runWavefront(plan, ops, plan.status.p, s);
             else runSweeps(plan, ops, s);
             RACE_CUDA(cudaEventRecord(ev[1], s));
             RACE_CUDA(cudaEventSynchronize(ev[1]));
@@ -1437,7 +1437,6 @@ int chooseSchedule(MpkPlan &plan, const race_operands &ops, cudaStream_t s) {
     int st = DEV_OK;
     RACE_CUDA(cudaMemcpyAsync(&st, plan.status.p, sizeof(int), cudaMemcpyDeviceToHost, s));
     RACE_CUDA(cudaStreamSynchronize(s));
-    RACE_CUDA(cudaMemsetAsync(plan.status.p, 0, sizeof(int), s));
     plan.chosen = (st == DEV_OK && ms[0] <= ms[1]) ? RACE_MPK_WAVEFRONT : RACE_MPK_SWEEPS;
     return plan.chosen;
 }
@@ -1446,7 +1445,6 @@ int chooseSchedule(MpkPlan &plan, const race_operands &ops, cudaStream_t s) {
 void runMpk(Engine &e, MpkPlan &plan, const race_operands &ops, int power) {
     if (power != plan.power) throw Error(RACE_ERR_INVALID_ARG, "power differs from the planned power");
     cudaStream_t s = e.stream;
-    e.lastStatus = nullptr;  // the plain launches wait for nothing
     if (plan.valType != RACE_VAL_F64) kToFloat<<<ceilDiv(ops.n, 256), 256, 0, s>>>((const double *)ops.x, plan.xf.p, ops.n);
     if (plan.stepped) {
         switch (plan.valType) {
@@ -1459,22 +1457,14 @@ void runMpk(Engine &e, MpkPlan &plan, const race_operands &ops, int power) {
         return;
     }
     const int sched = plan.schedule != RACE_MPK_AUTO ? plan.schedule : plan.chosen;
-    if (sched == RACE_MPK_WAVEFRONT) {
-        e.lastStatus = plan.status.p;
-        runWavefront(plan, ops, s);
-    } else if (sched == RACE_MPK_SWEEPS) {
-        runSweeps(plan, ops, s);
-    } else {
-        const int c = chooseSchedule(plan, ops, s);
-        if (plan.chosen == 0) {  // not timed (stream capture): run the default
-            if (c == RACE_MPK_WAVEFRONT) {
-                e.lastStatus = plan.status.p;
-                runWavefront(plan, ops, s);
-            } else {
-                runSweeps(plan, ops, s);
-            }
-        }
-    }
+    auto run = [&](int schedule) {
+        if (schedule == RACE_MPK_SWEEPS) return runSweeps(plan, ops, s);  // waits for nothing
+        e.noteWaits();
+        runWavefront(plan, ops, e.dStatus.p, s);
+    };
+    if (sched != RACE_MPK_AUTO) return run(sched);
+    const int c = chooseSchedule(plan, ops, s);
+    if (plan.chosen == 0) run(c);  // not timed (stream capture): run the default
 }
 
 // One plain SpMV x_{k+1} = A x_k on the registered SELL layout (the p-SpMV

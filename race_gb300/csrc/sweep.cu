@@ -869,22 +869,20 @@ void runSweep(Engine &e, FuncEntry &f, bool rev) {
     // GB300 beats the phase-by-phase executors by 9-37x on the 32^3 D2
     // SymmSpMV (0.010 ms against 0.089-0.77 ms per call)
     if (usesGather(e, f)) {
-        runGather(e, f, dir);
-        e.lastStatus = nullptr;  // no device waits
+        runGather(e, f, dir);  // waits for nothing
         return;
     }
     const bool waveMode = useWaveMode(e, f, dir);
+    e.noteWaits();
     // Gauss-Seidel and Kaczmarz: by dataflow, which replaces a grid barrier
     // per wave (or a leaf's serial walk per phase) by one L2 round trip per
     // dependent row, with the same sums; faster at every size measured
     // (4k rows to 100k, see flow.cu)
     if (f.flow[dir].ok) {
         runFlow(e, f, dir, !waveMode);
-        e.lastStatus = f.flowCtl.p;
         return;
     }
-    e.lastStatus = e.dStatus.p;
-    RACE_CUDA(cudaMemsetAsync(e.dStatus.p, 0, sizeof(int) * 4, e.stream));
+    RACE_CUDA(cudaMemsetAsync(e.dStatus.p + 2, 0, sizeof(int) * 2, e.stream));
     SweepArgs a{f.kernel, ops.rowPtr, ops.col, ops.val, ops.x, ops.b, nullptr, nullptr, nullptr, 0,
                 (unsigned *)(e.dStatus.p + 2), e.dStatus.p};
     a.midRow = midRowOf(e, f);

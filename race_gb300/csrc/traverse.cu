@@ -281,6 +281,8 @@ Engine::Engine(int nrow, int nthreads, int dist_, const int *rowPtr, const int *
     dKeysOut.alloc(nrow);
     dValsOut.alloc(nrow);
     dStatus.alloc(4);
+    RACE_CUDA(cudaMemsetAsync(dStatus.p, 0, sizeof(int) * 4, stream));
+    RACE_CUDA(cudaStreamSynchronize(stream));
     if (const char *st = getenv("RACE_GPU_MPK_STRIDE")) mpkStride = atoi(st) == 1 ? 1 : 2;
     if (const char *sp = getenv("RACE_GPU_MPK_SPLIT")) mpkSplit = std::max(0, atoi(sp));
     if (const char *o = getenv("RACE_GPU_MPK_ORDER")) mpkOrder = std::string(o) == "group" ? 1 : 0;

@@ -1,6 +1,7 @@
 """Waits of the dataflow sweeps that run out: with a limit of 64 polls a chain
 of thousands of dependent rows must end with RACE_ERR_TIMEOUT, and an engine
-with the default limit then computes the same function."""
+with the default limit then computes the same function. Launches behind the
+failed one do not hide it: it is reported once, also from replays of a graph."""
 import numpy as np
 import pytest
 
@@ -46,3 +47,52 @@ def test_a_wait_that_runs_out_ends_the_sweep(kernel, mode, vdt, monkeypatch):
         got[limit] = [rc.executeFunction(fid, rev) for rev in (False, True)]
     assert got == {"0": [TIMEOUT, TIMEOUT], "4194304": [0, 0]}
     assert bool(torch.isfinite(x).all())
+
+
+def _diagonal(rc, n):
+    """A Gauss-Seidel function whose rows wait for nothing: x = b / 2."""
+    i = torch.arange(n + 1, dtype=torch.int32, device="cuda")
+    x, b = torch.zeros(n, dtype=torch.float64, device="cuda"), torch.ones(n, dtype=torch.float64, device="cuda")
+    mat = ri.DeviceCsr(n, i, i[:-1].contiguous(), torch.full((n,), 2.0, dtype=torch.float64, device="cuda"))
+    return rc.registerFunction(ri.GS, ri.Operands(mat, x, b)), x, rc.registerFunction(ri.SPMV, ri.Operands(mat, b, x))
+
+
+@pytest.mark.gpu
+def test_a_failed_sweep_is_reported_behind_later_launches(monkeypatch):
+    monkeypatch.setenv("RACE_GPU_SWEEP_MAX_POLLS", "0")
+    A = _chain()
+    rc, P = _engine(A)
+    chain, _ = _function(rc, P, ri.GS)
+    diag, x, spmv = _diagonal(rc, A.n)
+    for later in ([(diag, False)], [(diag, False), (diag, True)], [(spmv, False)]):
+        assert rc.executeFunctionAsync(chain) == 0
+        for fid, rev in later:
+            assert rc.executeFunctionAsync(fid, rev) == 0
+        assert rc.getStatus() == TIMEOUT
+        assert rc.getStatus() == 0  # once
+        if later[0][0] == diag:
+            assert bool((x == 0).all())  # not run behind the failed one
+    x.zero_()
+    assert rc.executeFunction(diag) == 0 and bool((x == 0.5).all())
+    assert rc.executeFunctionAsync(chain) == 0
+    assert rc.executeFunction(spmv) == TIMEOUT  # a synchronous call reports it too
+    assert rc.executeFunction(spmv) == 0 and bool((x == 2.0).all())
+
+
+@pytest.mark.gpu
+def test_a_failed_replay_is_reported(monkeypatch):
+    monkeypatch.setenv("RACE_GPU_SWEEP_MAX_POLLS", "0")
+    A = _chain()
+    rc, P = _engine(A)
+    chain, _ = _function(rc, P, ri.GS)
+    torch.cuda.synchronize()
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    rc.setStream(stream)
+    with torch.cuda.graph(graph, stream=stream):
+        assert rc.executeFunctionAsync(chain) == 0
+    assert rc.getStatus() == 0
+    for _ in range(2):
+        with torch.cuda.stream(stream):
+            graph.replay()
+        assert rc.getStatus() == TIMEOUT
+        assert rc.getStatus() == 0
