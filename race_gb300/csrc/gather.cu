@@ -12,8 +12,8 @@
 // caller's, in place (they may change between calls). A row's own SymmSpMV
 // update (its diagonal, then its off-diagonal sum) stands in the list as its
 // diagonal's position with the sign bit, so that every step is the same fma.
-// Entries of b with more than kLongList updates, or whose own row is longer,
-// are folded by a warp each: it gathers 32 per lane and round while all lanes
+// Entries of b with many updates, or whose own row is long (foldLine), are
+// folded by a warp each: it gathers 32 per lane and round while all lanes
 // run the chain.
 //
 // What bounds it on GB300: the FP64 pipe (2 fma a cycle and SM: 32 us for the
@@ -28,6 +28,7 @@
 // us, SpMTV FP32 8,855 and 666 us.
 #include <algorithm>
 #include <climits>
+#include <utility>
 
 #include "engine.h"
 #include "sweep_ops.cuh"
@@ -37,8 +38,9 @@ namespace {
 
 constexpr int kGatherThreads = 128;
 constexpr int kGatherWarps = kGatherThreads / 32;
-// A thread's chain of this many updates takes as long as the rest of a launch;
-// beyond it a warp gathers for the chain (lists of a stencil stay below: 26).
+// Least number of updates of an entry that a warp gathers for (foldLine): a
+// thread's chain of that many takes as long as the rest of a small launch
+// (lists of a stencil stay below: 26).
 constexpr int kLongList = 96;
 
 struct GatherArgs {
@@ -266,6 +268,69 @@ void launchGatherK(const FuncEntry &f, const DevGather &g, cudaStream_t s) {
 
 }  // namespace
 
+// The number of updates (in an entry's list or its own row) above which a
+// warp folds the entry: kLongList, or more where so many entries are longer
+// that their folds fill the GPU. A warp's fold issues an instruction per
+// update, a thread's shares each with its 31 neighbours, so a matrix whose
+// rows are all long wants threads and a few hub rows want warps. Estimated
+// cycles of a line, whichever is longest: the folds on the GPU's 608 issue
+// queues (an FP64 instruction takes one for 64 cycles; FP32 with its loads
+// about 8), the longest fold of a warp (80 and 20 cycles an update) and of a
+// thread (140 and 80; measured on lists of up to 28k updates: own rows 100 and
+// 52, others' 183 and 105). Measured, 120k rows of 97 entries, with 96 as the
+// only line and now: SpMV FP64 608 and 45 us, FP32 65 and 37; SpMTV 618 and 44,
+// 131 and 35; 201 entries: 1,245 and 94, 108 and 85 (SpMV); the 50k-row
+// power-law graph keeps 96 (SpMV FP64 996 us, by threads alone 1,342; FP32 207
+// and 700).
+template <typename F>
+int foldLine(int n, bool f64, F &&lens) {
+    const double issue = (f64 ? 64.0 : 8.0) / 608, warpChain = f64 ? 80 : 20, threadChain = f64 ? 140 : 80;
+    struct Line {
+        double issue, chain;      // estimated cycles
+        long long slots, updates; // of the padded lists and without padding
+        int longest;
+        double cycles() const { return std::max(issue, chain); }
+    };
+    auto estimate = [&](int line) {
+        long long folds = 0, slots = 0, updates = 0, warpMost = 0, threadMost = 0;
+        int longest = 0;
+        for (int c = 0; c < n; c += 32) {
+            int own = 0, list = 0;
+            for (int y = c; y < std::min(n, c + 32); ++y) {
+                const auto [o, l] = lens(y);
+                longest = std::max(longest, std::max(o, l));
+                updates += l;
+                if (std::max(o, l) > line) {
+                    folds += (long long)o + l;
+                    warpMost = std::max(warpMost, (long long)o + l);
+                } else {
+                    own = std::max(own, o);
+                    list = std::max(list, l);
+                    threadMost = std::max(threadMost, (long long)o + l);
+                }
+            }
+            folds += own + list;
+            slots += 32LL * list;
+        }
+        return Line{issue * folds, std::max(warpChain * warpMost, threadChain * threadMost), slots, updates, longest};
+    };
+    int line = kLongList;
+    const Line first = estimate(line);
+    double best = first.cycles();
+    // only the issue queues' time can shrink
+    if (first.issue <= first.chain) return line;
+    for (int next = line; next < first.longest;) {
+        next = next & (next - 1) ? next / 3 * 4 : next / 2 * 3;  // 128, 192, 256, 384, ...
+        const Line e = estimate(next);
+        if (e.slots > 4 * e.updates) break;  // lists are padded to their chunk's longest
+        if (e.cycles() < 0.8 * best) {
+            best = e.cycles();
+            line = next;
+        }
+    }
+    return line;
+}
+
 // The device lists of one direction (SpMV: of both) from the host CRS.
 void buildGather(Engine &e, FuncEntry &f, int dir, const std::vector<int> &rp, const std::vector<int> &cl) {
     DevGather &g = f.gather[dir];
@@ -278,24 +343,35 @@ void buildGather(Engine &e, FuncEntry &f, int dir, const std::vector<int> &rp, c
     std::vector<int> len(std::max(n, 1), 0), longY;
     std::vector<long long> listOff(std::max(C, 1), 0);
     long long listSlots = 0;
-    for (int c = 0; c < C; ++c) {
-        int width = 0;
-        for (int y = 32 * c; y < std::min(n, 32 * c + 32); ++y) {
-            const int rowLen = rp[y + 1] - rp[y], ownLen = own ? std::max(0, rowLen - first) : 0;
-            int cnt = lists ? gp.ptr[y + 1] - gp.ptr[y] : 0;
-            if (std::max(cnt, ownLen) > kLongList) {
-                len[y] = -1;
-                longY.push_back(y);
-                continue;
+    auto lens = [&](int y) {
+        return std::pair<int, int>(own ? std::max(0, rp[y + 1] - rp[y] - first) : 0, lists ? gp.ptr[y + 1] - gp.ptr[y] : 0);
+    };
+    auto cut = [&](int line) {
+        longY.clear();
+        listSlots = 0;
+        for (int c = 0; c < C; ++c) {
+            int width = 0;
+            for (int y = 32 * c; y < std::min(n, 32 * c + 32); ++y) {
+                auto [ownLen, cnt] = lens(y);
+                if (std::max(cnt, ownLen) > line) {
+                    len[y] = -1;
+                    longY.push_back(y);
+                    continue;
+                }
+                if (first && rp[y] == rp[y + 1]) {  // its own update is left out (kListLayout)
+                    for (int i = gp.ptr[y]; i < gp.ptr[y + 1]; ++i) cnt -= gp.entry[i] < 0;
+                }
+                len[y] = cnt;
+                width = std::max(width, cnt);
             }
-            if (first && rowLen == 0) {  // its own update is left out (kListLayout)
-                for (int i = gp.ptr[y]; i < gp.ptr[y + 1]; ++i) cnt -= gp.entry[i] < 0;
-            }
-            len[y] = cnt;
-            width = std::max(width, cnt);
+            listOff[c] = listSlots;
+            listSlots += 32LL * ((width + 3) & ~3);
         }
-        listOff[c] = listSlots;
-        listSlots += 32LL * ((width + 3) & ~3);
+    };
+    cut(kLongList);
+    if (!longY.empty()) {
+        const int line = foldLine(n, f.ops.vec_type == RACE_VAL_F64, lens);
+        if (line != kLongList) cut(line);
     }
     // the longest first: a warp each, and the longest bounds the launch
     auto work = [&](int y) {
