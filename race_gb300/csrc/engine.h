@@ -164,7 +164,7 @@ struct DevFlow {
 // layout per 32 entries of b (gather.cu), built at the first gather-mode call
 // (SpMV: at registration, in the forward direction's place).
 struct DevGather {
-    bool built = false;
+    bool built = false, plain = false;  // plain: kGatherPlain, no layout
     int numLong = 0;
     DevBuf<int> mem;  // holds all of the tables below
     long long *listOff = nullptr;

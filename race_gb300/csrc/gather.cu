@@ -215,6 +215,40 @@ __global__ void __launch_bounds__(kShortThreads, kShortBlocks)
     if (numLong && blockIdx.x == gridDim.x - 1) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// Large matrices with short rows: a thread per entry of b on the caller's CRS
+// and the plain lists. Nothing of a short list is padding there and twice as
+// many threads are resident, which decides where loads in flight do (gatherPlain).
+template <typename VT, typename XT, int KER>
+__global__ void __launch_bounds__(256)
+    kGatherPlain(int n, const int *__restrict__ ptr, const int *__restrict__ entry, const int *__restrict__ src,
+                 const int *__restrict__ rowPtr, const int *__restrict__ col, const VT *__restrict__ val,
+                 const XT *__restrict__ x, XT *__restrict__ b) {
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    for (long long y = (long long)blockIdx.x * blockDim.x + threadIdx.x; y < n; y += stride) {
+        if constexpr (KER == RACE_K_SPMV) {
+            XT t = XT(0);
+            for (int j = rowPtr[y]; j < rowPtr[y + 1]; ++j) t = mac(ld<VT, XT>(val, j), x[col[j]], t);
+            b[y] = t;
+        } else {
+            XT acc = b[y];
+            for (int k = ptr[y]; k < ptr[y + 1]; ++k) {
+                const int e = entry[k];
+                if (KER == RACE_K_SPMTV || e >= 0) {  // another row's update
+                    acc = mac(ld<VT, XT>(val, e), x[src[k]], acc);
+                    continue;
+                }
+                const int s = rowPtr[y], end = rowPtr[y + 1];
+                if (end == s) continue;  // a row without entries has no update of its own
+                acc = mac(ld<VT, XT>(val, s), x[y], acc);
+                XT t = XT(0);
+                for (int j = s + 1; j < end; ++j) t = mac(ld<VT, XT>(val, j), x[col[j]], t);
+                acc += t;
+            }
+            b[y] = acc;
+        }
+    }
+}
+
 // Lists of one chunk's entries of b from GatherPlan's, a warp per chunk.
 __global__ void kListLayout(int n, int numChunks, const int *__restrict__ len, const int *__restrict__ ptr,
                             const int *__restrict__ entry, const int *__restrict__ src,
@@ -239,6 +273,12 @@ template <typename VT, typename XT, int KER>
 void launchGather(const FuncEntry &f, const DevGather &g, cudaStream_t s) {
     const race_operands &o = f.ops;
     if (o.n == 0) return;
+    if (g.plain) {
+        kGatherPlain<VT, XT, KER><<<std::min(ceilDiv(o.n, 256), 152 * 16), 256, 0, s>>>(
+            o.n, g.ptr, g.entry, g.row, o.rowPtr, o.col, (const VT *)o.val, (const XT *)o.x, (XT *)o.b);
+        RACE_CUDA(cudaGetLastError());
+        return;
+    }
     const GatherArgs a{o.n,     g.numLong,   o.rowPtr,    o.col,       o.val,     o.x,     o.b,       g.len,
                        g.listOff, g.listPos, g.listSrc, g.longY, g.ptr, g.entry, g.row};
     if (a.numLong) {
@@ -331,6 +371,25 @@ int foldLine(int n, bool f64, F &&lens) {
     return line;
 }
 
+// Whether kGatherPlain runs a matrix without long entries: from half a million
+// rows on (a grid of resident threads then takes more than one turn) and up to
+// twelve updates per entry of b. Measured, microseconds with kGather and with
+// kGatherPlain, 5-, 7- and 9-point stencils of about 700k rows, and of 1.4 to 2
+// million: SpMV FP64 10.6 and 10.3, 14.4 and 12.4, 18.5 and 16.4; 38 and 29, 43
+// and 35, 40 and 38; FP32 8.3 and 6.3, 10.4 and 8.3, 10.3 and 10.3; 27 and 17,
+// 33 and 24, 27 and 25. SpMTV FP64 25 and 16, 27 and 19, 37 and 30; 62 and 43,
+// 59 and 51, 62 and 58; FP32 14.5 and 12.2, 16.5 and 14.5, 23 and 19; 44 and
+// 32, 43 and 38, 45 and 40. SymmSpMV FP64 23 and 20, 34 and 31, 41 and 34; 69
+// and 50, 77 and 62, 73 and 57; FP32 16.5 and 14.5, 20.0 and 20.6, 20.7 and
+// 20.7; 51 and 39, 52 and 45, 47 and 41 (so FP32 with more than six updates
+// waits for a million rows). With 360k rows it is the other way round for 9
+// points (SymmSpMV FP64 23 and 25, SpMTV FP32 11.8 and 14.2), and for 27-point
+// rows at every size (SymmSpMV FP64 753k rows 93 and 144).
+bool gatherPlain(int kernel, bool f64, int n, double updates) {
+    const bool late = kernel == RACE_K_SYMMSPMV && !f64 && updates > 6;
+    return n >= (late ? 1 << 20 : 1 << 19) && updates <= 12;
+}
+
 // The device lists of one direction (SpMV: of both) from the host CRS.
 void buildGather(Engine &e, FuncEntry &f, int dir, const std::vector<int> &rp, const std::vector<int> &cl) {
     DevGather &g = f.gather[dir];
@@ -340,13 +399,15 @@ void buildGather(Engine &e, FuncEntry &f, int dir, const std::vector<int> &rp, c
     cudaStream_t s = e.stream;
     GatherPlan gp;
     if (lists) gp = buildGatherPlan(f.kernel, n, rp.data(), cl.data(), e.phases[dir]);
-    std::vector<int> len(std::max(n, 1), 0), longY;
-    std::vector<long long> listOff(std::max(C, 1), 0);
+    std::vector<int> len, longY;
+    std::vector<long long> listOff;
     long long listSlots = 0;
     auto lens = [&](int y) {
         return std::pair<int, int>(own ? std::max(0, rp[y + 1] - rp[y] - first) : 0, lists ? gp.ptr[y + 1] - gp.ptr[y] : 0);
     };
     auto cut = [&](int line) {
+        len.assign(std::max(n, 1), 0);
+        listOff.assign(std::max(C, 1), 0);
         longY.clear();
         listSlots = 0;
         for (int c = 0; c < C; ++c) {
@@ -368,10 +429,15 @@ void buildGather(Engine &e, FuncEntry &f, int dir, const std::vector<int> &rp, c
             listSlots += 32LL * ((width + 3) & ~3);
         }
     };
-    cut(kLongList);
-    if (!longY.empty()) {
-        const int line = foldLine(n, f.ops.vec_type == RACE_VAL_F64, lens);
-        if (line != kLongList) cut(line);
+    const bool f64 = f.ops.vec_type == RACE_VAL_F64;
+    int most = 0;
+    for (int y = 0; own && y < n; ++y) most = std::max(most, rp[y + 1] - rp[y] - first);
+    for (int y = 0; lists && y < n; ++y) most = std::max(most, gp.ptr[y + 1] - gp.ptr[y]);
+    const double updates = ((own ? (double)rp[n] - first * (double)n : 0.0) + gp.entry.size()) / std::max(n, 1);
+    g.plain = most <= kLongList && gatherPlain(f.kernel, f64, n, updates);
+    if (!g.plain) {
+        const int line = most > kLongList ? foldLine(n, f64, lens) : kLongList;
+        cut(line);
     }
     // the longest first: a warp each, and the longest bounds the launch
     auto work = [&](int y) {
@@ -409,7 +475,7 @@ void buildGather(Engine &e, FuncEntry &f, int dir, const std::vector<int> &rp, c
         put(g.entry, gp.entry.data(), sizeof(int) * entries);
         put(g.row, gp.row.data(), sizeof(int) * entries);
         put(g.listOff, listOff.data(), sizeof(long long) * listOff.size());
-        if (C > 0)
+        if (C > 0 && !g.plain)
             kListLayout<<<ceilDiv(32LL * C, 256), 256, 0, s>>>(n, C, g.len, g.ptr, g.entry, g.row, f.ops.rowPtr, g.listOff,
                                                                g.listPos, g.listSrc);
     }
