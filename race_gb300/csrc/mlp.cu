@@ -18,8 +18,8 @@
 // Networks that do not fit in shared memory take the tiles (kForward: a block
 // takes a few rows through all layers, weights in tiles fetched one ahead
 // across the layer boundaries; kBackward), networks wider than kFusedDim or
-// deeper than kFusedLayers the products one by one (kGemm: 32 x 32 output
-// tiles, 16-deep k slices).
+// deeper than kFusedLayers, and wide ones with few rows (byProducts), the
+// products one by one (kGemm: 32 x 32 output tiles, 16-deep k slices).
 // Each output sums its terms in order with fmaf in either form, so results do
 // not depend on the grid; above kGradRows rows the weight gradients are summed
 // in chunks of rows, added in order (kGradReduce). The loss reduction runs in
@@ -647,7 +647,7 @@ struct Mlp {
     DevBuf<float> acts, deltas;  // activations per layer, gradients of them (one product at a time: two of the widest)
     DevBuf<float> part;          // gradients of chunks of rows
     float *hostGrads = nullptr;  // pinned: gradients and loss on their way to the caller
-    bool fused = false;          // one kernel per pass (else one per product)
+    bool fused = false;          // has passes of one kernel (else one kernel per product)
     unsigned sharedAllowed = 0;  // allowShared's kernels, a bit each
     int batchCap = 0;
     long long steps = 0;
@@ -697,7 +697,7 @@ struct Mlp {
             widest = std::max(widest, (size_t)B * std::max(dimOut[l], dimIn[l]));
         }
         acts.alloc(total);
-        deltas.alloc(fused ? total : 2 * widest);
+        deltas.alloc(fused ? std::max(total, 2 * widest) : 2 * widest);  // fused networks: both forms (byProducts)
         if (fused && gradChunks(B) > 1) part.ensure(gradStride() * gradChunks(B));
         batchCap = B;
     }
@@ -784,9 +784,31 @@ struct Mlp {
         RACE_CUDA(cudaStreamIsCapturing(s, &st));
         return st != cudaStreamCaptureStatusNone;
     }
+    // Whether a batch runs one kernel per product: networks that no fused pass
+    // takes, and wide ones with few rows. A fused block of a few rows goes
+    // through all weights by itself, 1.2 us a tile; a product's blocks share
+    // them and take 0.083 us a term of their sums (0.072 up to one row of
+    // blocks, 1.2 times that where they do not fit on the GPU at once).
+    // Measured, outputs and gradients, fused / by products, microseconds:
+    // 34-1024-1024-1024-1, 64 rows 341 and 701 / 255 and 469, 256 rows 342 and
+    // 762 / 309 and 658, 320 rows 389 and 870 / 412 and 866; 34-768-768-768-1,
+    // 16 rows 197 and 395 / 173 and 314, 256 rows 200 and 441 / 239 and 512;
+    // 34-512-512-512-1, 64 rows 97 and 193 / 136 and 263.
+    bool byProducts(int B) const {
+        if (!fused) return true;
+        if (B > 256 || residentBytes(rowsPerBlock(B)) <= kResidentBytes) return false;
+        long long tiles = 0, terms = 0, blocks = 0;
+        for (int l = 0; l < layers(); ++l) {
+            tiles += (long long)ceilDiv(dimOut[l], kTileN) * ceilDiv(dimIn[l], kTileK);
+            terms += dimIn[l];
+            blocks = std::max(blocks, (long long)ceilDiv(dimOut[l], kT) * ceilDiv(B, kT));
+        }
+        return (B <= kT ? 0.072 : 0.083) * terms * (blocks > kResidentSms ? 1.2 : 1.0) < 1.2 * tiles;
+    }
     // outputs only, to Y
     void predict(const float *X, int B, float *Y, cudaStream_t s) {
-        if (!fused) {
+        // (a capture cannot allocate the products' workspace; the fused pass needs none)
+        if (!fused || (byProducts(B) && (B <= batchCap || !capturing(s)))) {
             const float *y = forward(X, B, s);
             RACE_CUDA(cudaMemcpyAsync(Y, y, sizeof(float) * B * out, cudaMemcpyDeviceToDevice, s));
             return;
@@ -855,9 +877,13 @@ struct Mlp {
         }
         return acts.p + actOff(layers(), B);
     }
-    // loss and gradients of the MSE against targets T (B x out)
-    void lossGrad(const float *X, const float *T, int B, float *host, cudaStream_t s) {
-        if (fused) return lossGradFused(X, T, B, host, s);
+    // loss and gradients of the MSE against targets T (B x out); returns
+    // whether the kernels wrote them to host too
+    bool lossGrad(const float *X, const float *T, int B, float *host, cudaStream_t s) {
+        if (!byProducts(B)) {
+            lossGradFused(X, T, B, host, s);
+            return host != nullptr;
+        }
         float *y = forward(X, B, s);
         float *d = deltas.p, *dNext = deltas.p + deltas.n / 2;
         kMse<<<1, 256, 0, s>>>(B * out, y, T, d, loss());
@@ -876,6 +902,7 @@ struct Mlp {
                 std::swap(d, dNext);
             }
         }
+        return false;
     }
     void adam(float lr, float b1, float b2, float eps, cudaStream_t s) {
         ++steps;
@@ -972,9 +999,9 @@ int race_mlp_loss_grad(race_mlp *h, const float *X, const float *T, int batch, f
         const bool wanted = loss_host || grad_host;
         if (wanted && !net.hostGrads)
             RACE_CUDA(cudaMallocHost((void **)&net.hostGrads, sizeof(float) * (net.numParams + 1)));
-        net.lossGrad(X, T, batch, grad_host ? net.hostGrads : nullptr, s);
+        const bool there = net.lossGrad(X, T, batch, grad_host ? net.hostGrads : nullptr, s);
         if (!wanted) return;
-        if (!net.fused || !grad_host) {
+        if (!there) {
             const size_t first = grad_host ? 0 : net.numParams;
             RACE_CUDA(cudaMemcpyAsync(net.hostGrads + first, net.grads.p + first,
                                       sizeof(float) * (net.numParams + 1 - first), cudaMemcpyDeviceToHost, s));
