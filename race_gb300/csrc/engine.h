@@ -47,7 +47,7 @@ struct MpkPlan {
     DevBuf<unsigned char> hubVal;  // hub entries (type valType)
     DevBuf<int> hubCol;
     // the hub rows as work of the plain SpMV (mpk.cu HubWork)
-    int hubBig = 0, hubWork = 0;
+    int hubBig = 0, hubWork = 0, hubLongest = 0;
     DevBuf<int> hubWorkRow, hubSegFirst, hubCount;
     DevBuf<double> hubSegPart;
     DevBuf<float> hubBigVal;    // FP32/BF16: values of the rows that a block sums

@@ -72,6 +72,9 @@ constexpr int kSmallWarpsPerSm = 32;
 // (two tiles at least). The longest row bounds a power-law matrix, so the line
 // hardly matters: 110 and 116 us at 1,024 and 4,096 for the graph below.
 constexpr int kHubBlockLen = 1024;
+// Longest FP32/BF16 hub row that a warp of the striding kernel takes
+// (spmvForm).
+constexpr int kHubStrideLen = 8192;
 
 namespace {
 
@@ -567,19 +570,19 @@ __device__ __forceinline__ void putRow(float v, int r, int k, int n, double *x, 
 // FP64: one segment of a hub row by one warp. The warp that finishes the
 // row's last segment adds them up as hubSum does and leaves the row's counter
 // at zero for the next launch. FP32/BF16: one shorter hub row by one warp.
-template <typename VT, typename AT>
+template <typename VT, typename AT, int U>
 __device__ __forceinline__ void hubTask(const SellView &m, const HubWork &hw, int i, int k, int n, const AT *xin,
                                         double *x, float *xf) {
     const int lane = threadIdx.x & 31;
     if constexpr (sizeof(VT) != 8) {
         const int h = hw.hub[hw.big + i];
-        const AT t = hubSegment<VT, AT, 8>(m, m.hubPtr[h], m.hubPtr[h + 1], xin);
+        const AT t = hubSegment<VT, AT, U>(m, m.hubPtr[h], m.hubPtr[h + 1], xin);
         if (lane == 0) putRow(t, m.hubRow[h], k, n, x, xf);
     } else {
         const int h = hw.hub[i];
         const int first = hw.first[h], segs = hw.first[h + 1] - first;
         const int beg = m.hubPtr[h] + (i - first) * kMpkHubSeg;
-        AT t = hubSegment<VT, AT, 8>(m, beg, min(m.hubPtr[h + 1], beg + kMpkHubSeg), xin);
+        AT t = hubSegment<VT, AT, U>(m, beg, min(m.hubPtr[h + 1], beg + kMpkHubSeg), xin);
         if (segs > 1) {
             AT *part = (AT *)hw.part;
             int last = 0;
@@ -694,14 +697,38 @@ __device__ __forceinline__ void hubBlock(const SellView &m, int h, const float *
 // with 32 registers and 8 blocks an SM. Odd powers run from the last chunk to
 // the first: what the L2 still holds of a matrix that does not fit is its end
 // (27-point 97x113x89, FP32: 162 MB a power, 305 us with all powers forward).
-template <typename VT, bool C16>
+// Hub rows (FP64: their segments) come first, a warp each (STRIDE_HUBS), or,
+// where a row of some thousand entries lasts as long as a warp's chunks, to
+// warps that take nothing else (STRIDE_APART). Entries three at a time, to stay
+// within the chunks' registers.
+enum Form : int { ONE_PIECE = -1, STRIDE = 0, STRIDE_HUBS = 1, STRIDE_APART = 2 };
+
+template <typename VT, int FORM, bool C16>
 __global__ void __launch_bounds__(kWarpThreads, kSpmvMinBlocks<VT>)
-    kSpmvSell(SellView m, int numChunks, int n, int k, double *x, float *xf) {
+    kSpmvSell(SellView m, HubWork hw, int numChunks, int n, int k, double *x, float *xf) {
+    using AT = typename std::conditional<sizeof(VT) == 8, double, float>::type;
     pdlTrigger();
     pdlWait();
-    const int nw = gridDim.x * (blockDim.x >> 5);
-    for (int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < numChunks; i += nw)
-        chunkRow<VT, false, C16>(m, k & 1 ? numChunks - 1 - i : i, k, n, x, xf, 0);
+    const int nw = gridDim.x * (blockDim.x >> 5), hubs = FORM == STRIDE ? 0 : hw.big + hw.num;
+    int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), step = nw;
+    auto hubRow = [&](int h) {
+        const AT *xin;
+        if constexpr (sizeof(VT) == 8) xin = x + (size_t)k * n;
+        else xin = xf + (size_t)k * n;
+        hubTask<VT, AT, 3>(m, hw, h - hw.big, k, n, xin, x, xf);
+    };
+    if constexpr (FORM == STRIDE_APART) {
+        if (i < hubs) return hubRow(i);
+        step = nw - hubs;
+    }
+    for (; i < hubs + numChunks; i += step) {
+        if (FORM == STRIDE_HUBS && i < hubs) {
+            hubRow(i);
+            continue;
+        }
+        const int c = i - hubs;
+        chunkRow<VT, false, C16>(m, k & 1 ? numChunks - 1 - c : c, k, n, x, xf, 0);
+    }
 }
 
 // kSpmvSellSmall: one piece of work a warp, for matrices of at most
@@ -729,7 +756,7 @@ __global__ void __launch_bounds__(kWarpThreads, kSmallWarpsPerSm * 32 / kWarpThr
         }
         if (c < hw.num) {
             pdlWait();
-            hubTask<VT, AT>(m, hw, c, k, n, xin, x, xf);
+            hubTask<VT, AT, 8>(m, hw, c, k, n, xin, x, xf);
             return;
         }
         c -= hw.num;
@@ -1057,6 +1084,7 @@ std::unique_ptr<MpkPlan> buildMpkPlan(Engine &e, const race_operands &ops, int p
                 segFirst.push_back(segFirst.back() + hubLen(work[plan->hubBig]));
         }
         plan->hubWork = (int)work.size() - plan->hubBig;
+        for (int h = 0; h < H; ++h) plan->hubLongest = std::max(plan->hubLongest, hubLen(h));
         plan->hubWorkRow.upload(work.data(), work.size(), s);
         plan->hubSegFirst.upload(segFirst.data(), segFirst.size(), s);
         if (ops.val_type == RACE_VAL_F64) {
@@ -1297,6 +1325,34 @@ void launchMpkSteps(const MpkPlan &p, int n, double *x, cudaStream_t s) {
     }
 }
 
+// The plain SpMV's kernel of a plan. One piece a warp for small matrices, and
+// for large ones whose hub rows decide: FP64 above 0.25 % of the entries in
+// them, FP32 and BF16 above 1 %, or a row too long for a warp beside the chunks
+// (750 entries per kSmallWarpsPerSm chunks an SM, 8,192 at most). Measured, p =
+// 4, one piece / striding: 27-point 90^3 with 30 rows of 600 entries FP64 207
+// and 180, BF16 156 and 101 us, 110^3 with one of 3,000 FP32 253 and 198, BF16
+// 299 and 168; the other way 62^3 with 300 rows of 400 FP64 80 and 104, 75^3
+// with one of 3,000 FP32 73 and 102, the 300k-row power-law graph FP64 210 and
+// 338.
+Form spmvForm(const MpkPlan &p) {
+    const long long line = kSmallWarpsPerSm * devSms(), entries = (long long)p.hubCol.n;
+    if (p.numChunks <= line) return ONE_PIECE;
+    if (p.numHubs == 0) return STRIDE;
+    if (p.valType == RACE_VAL_F64) return entries * 400 <= p.sellSlots ? STRIDE_HUBS : ONE_PIECE;
+    if (entries * 100 > p.sellSlots) return ONE_PIECE;
+    if (p.hubBig == 0) return STRIDE_HUBS;
+    // (few enough hub rows for most warps of any grid of one block an SM)
+    return p.hubLongest <= kHubStrideLen && line * p.hubLongest <= 750LL * p.numChunks && p.numHubs <= 4 * devSms()
+               ? STRIDE_APART : ONE_PIECE;
+}
+
+template <typename VT, int FORM, bool C16>
+void launchStriding(const MpkPlan &p, const HubWork &hw, cudaLaunchConfig_t &cfg, int n, int k, double *x) {
+    static const int resident = residentBlocks(kSpmvSell<VT, FORM, C16>, kWarpThreads);
+    cfg.gridDim = dim3(std::min(resident, (int)cfg.gridDim.x));
+    RACE_CUDA(cudaLaunchKernelEx(&cfg, kSpmvSell<VT, FORM, C16>, viewOf(p), hw, p.numChunks, n, k, x, p.xf.p));
+}
+
 template <typename VT, bool HUBS, bool C16>
 void launchSpmvSellK(const MpkPlan &p, int n, int k, double *x, cudaStream_t s) {
     cudaLaunchAttribute at{};
@@ -1307,16 +1363,20 @@ void launchSpmvSellK(const MpkPlan &p, int n, int k, double *x, cudaStream_t s) 
     cfg.stream = s;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
+    const HubWork hw{p.hubBig, p.hubWork, p.hubWorkRow.p, p.hubSegFirst.p, p.hubCount.p, p.hubSegPart.p, p.hubBigVal.p};
     const int blocks = std::max(1, ceilDiv((long long)p.hubWork + p.numChunks, kWarpThreads / 32));
-    if (HUBS || p.numChunks <= kSmallWarpsPerSm * devSms()) {
-        const HubWork hw{p.hubBig, p.hubWork, p.hubWorkRow.p, p.hubSegFirst.p, p.hubCount.p, p.hubSegPart.p, p.hubBigVal.p};
+    cfg.gridDim = dim3(blocks);
+    const Form form = spmvForm(p);
+    if (form == ONE_PIECE) {
         cfg.gridDim = dim3(p.hubBig + blocks);
         RACE_CUDA(cudaLaunchKernelEx(&cfg, kSpmvSellSmall<VT, HUBS, C16>, viewOf(p), hw, p.numChunks, n, k, x, p.xf.p));
-        return;
+    } else if constexpr (!HUBS) {
+        launchStriding<VT, STRIDE, C16>(p, hw, cfg, n, k, x);
+    } else if (form == STRIDE_HUBS) {
+        launchStriding<VT, STRIDE_HUBS, C16>(p, hw, cfg, n, k, x);
+    } else if constexpr (sizeof(VT) != 8) {
+        launchStriding<VT, STRIDE_APART, C16>(p, hw, cfg, n, k, x);
     }
-    static const int resident = residentBlocks(kSpmvSell<VT, C16>, kWarpThreads);
-    cfg.gridDim = dim3(std::min(resident, blocks));
-    RACE_CUDA(cudaLaunchKernelEx(&cfg, kSpmvSell<VT, C16>, viewOf(p), p.numChunks, n, k, x, p.xf.p));
 }
 
 template <typename VT>
@@ -1336,10 +1396,11 @@ template <typename VT, bool HUBS, bool C16>
 void loadSchedulesK(const MpkPlan &p) {
     cudaFuncAttributes fa;
     RACE_CUDA(cudaFuncGetAttributes(&fa, kMpk<VT, HUBS, C16>));
-    if (HUBS || p.numChunks <= kSmallWarpsPerSm * devSms())
-        RACE_CUDA(cudaFuncGetAttributes(&fa, kSpmvSellSmall<VT, HUBS, C16>));
-    else
-        RACE_CUDA(cudaFuncGetAttributes(&fa, kSpmvSell<VT, C16>));
+    const Form form = spmvForm(p);
+    if (form == ONE_PIECE) RACE_CUDA(cudaFuncGetAttributes(&fa, kSpmvSellSmall<VT, HUBS, C16>));
+    else if constexpr (!HUBS) RACE_CUDA(cudaFuncGetAttributes(&fa, kSpmvSell<VT, STRIDE, C16>));
+    else if (form == STRIDE_HUBS) RACE_CUDA(cudaFuncGetAttributes(&fa, kSpmvSell<VT, STRIDE_HUBS, C16>));
+    else if constexpr (sizeof(VT) != 8) RACE_CUDA(cudaFuncGetAttributes(&fa, kSpmvSell<VT, STRIDE_APART, C16>));
 }
 
 template <typename VT>
