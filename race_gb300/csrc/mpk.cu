@@ -558,6 +558,70 @@ __device__ __forceinline__ AT sellRowAhead(const VT *__restrict__ val, long long
     return t;
 }
 
+// The values of an entry group as loaded; get() decodes them.
+template <typename VT>
+struct GroupWords {
+    VT v[4];
+    __device__ __forceinline__ void load(const VT *p) { groupVals<false>(p, 0, v, 0); }
+    __device__ __forceinline__ void get(VT to[4]) const { to[0] = v[0], to[1] = v[1], to[2] = v[2], to[3] = v[3]; }
+};
+template <>
+struct GroupWords<__nv_bfloat16> {
+    uint2 a;
+    __device__ __forceinline__ void load(const __nv_bfloat16 *p) { a = *(const uint2 *)p; }
+    __device__ __forceinline__ void get(float to[4]) const {
+        to[0] = __uint_as_float(a.x << 16);
+        to[1] = __uint_as_float(a.x & 0xffff0000u);
+        to[2] = __uint_as_float(a.y << 16);
+        to[3] = __uint_as_float(a.y & 0xffff0000u);
+    }
+};
+
+// sellRowAhead on the 16-bit columns of a matrix with hub rows, whose other
+// rows are up to 256 entries long: columns and values are kept as loaded until
+// their round, since decoding one waits for its load, a round too early
+// (power-law graph of 5,000 rows, p = 4: BF16 125 and 78 us, FP64 114 and 96).
+// The two groups of a stencil's row are loaded and decoded before x may be read
+// and stay with sellRowAhead (7-point 32^3 13.7 us, 13.9 and more here).
+template <typename VT, typename AT>
+__device__ __forceinline__ AT sellRowLate(const VT *__restrict__ val, const void *col, long long off, int4 b, int len,
+                                          const AT *x) {
+    AT t = AT(0), xv[4] = {AT(0), AT(0), AT(0), AT(0)};
+    GroupWords<VT> w{}, wn{};
+    uint2 c = make_uint2(0, 0), cn = c;
+    const unsigned short *cols = (const unsigned short *)col + off;
+    auto gather = [&](const uint2 &q, int left, AT (&to)[4]) {
+        if (left > 0) to[0] = x[col16Of(q.x & 0xffffu, b)];
+        if (left > 1) to[1] = x[col16Of(q.x >> 16, b)];
+        if (left > 2) to[2] = x[col16Of(q.y & 0xffffu, b)];
+        if (left > 3) to[3] = x[col16Of(q.y >> 16, b)];
+    };
+    if (len > 0) {
+        w.load(val + off);
+        c = *(const uint2 *)cols;
+    }
+    if (len > 4) cn = *(const uint2 *)(cols + 128);
+    pdlWait();
+    gather(c, len, xv);
+    for (int j = 0; j < len; j += 4) {
+        AT v[4], xn[4] = {AT(0), AT(0), AT(0), AT(0)};
+        if (j + 4 < len) {
+            gather(cn, len - j - 4, xn);
+            wn.load(val + off + 32LL * (j + 4));
+            if (j + 8 < len) cn = *(const uint2 *)(cols + 32LL * (j + 8));
+        }
+        w.get(v);
+        t = fma(v[0], xv[0], t);
+        if (len - j > 1) t = fma(v[1], xv[1], t);
+        if (len - j > 2) t = fma(v[2], xv[2], t);
+        if (len - j > 3) t = fma(v[3], xv[3], t);
+        w = wn;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) xv[q] = xn[q];
+    }
+    return t;
+}
+
 // Result of row r at power k -> k+1 (FP32/BF16 also to the FP64 powers).
 __device__ __forceinline__ void putRow(double v, int r, int k, int n, double *x, float *) {
     x[(size_t)(k + 1) * n + r] = v;
@@ -772,8 +836,10 @@ __global__ void __launch_bounds__(kWarpThreads, kSmallWarpsPerSm * 32 / kWarpThr
     AT t;
     if constexpr (C16) {
         const int4 b = m.chunkBase[c];
-        t = b.x >= 0 ? sellRowAhead<VT, AT, true>(val, off, m.col16, off, b, len, xin)
-                     : sellRowAhead<VT, AT, false>(val, off, m.wideCol, (long long)b.y + 4 * lane, b, len, xin);
+        if (HUBS && b.x >= 0) t = sellRowLate<VT, AT>(val, m.col16, off, b, len, xin);
+        else
+            t = b.x >= 0 ? sellRowAhead<VT, AT, true>(val, off, m.col16, off, b, len, xin)
+                         : sellRowAhead<VT, AT, false>(val, off, m.wideCol, (long long)b.y + 4 * lane, b, len, xin);
     } else {
         t = sellRowAhead<VT, AT, false>(val, off, m.col, off, make_int4(0, 0, 0, 0), len, xin);
     }
