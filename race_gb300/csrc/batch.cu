@@ -71,6 +71,16 @@ int blockMaxRows(int nrhs, int vecType) {
     const int rows = 4096 / (nrhs * (vecType == RACE_VAL_F64 ? 8 : 4));
     return std::min(128, std::max(32, rows & ~31));
 }
+// Whether a batch's items mostly wait for one another (kMpkBlock, FEW): up to
+// three chunks for four warps, and with long rows, whose chain of loads is the
+// item's time, up to four chunks a warp. Measured, the other form / FEW, p = 8
+// unless noted: 7-point 40^3, one FP64 right-hand side (2,000 chunks) 120 and
+// 101 us; 9-point 300^2, 8 FP32 ones (5,600) 108 and 101; 27-point 50^3, one FP64
+// (3,900) 385 and 298, 16 FP32 (15,600) 319 and 292; 5- and 9-point 250^2, 16
+// FP32, p = 4 (8,100) 41 and 43; 16 of 100^2 to 500^2, 8 BF16, p = 4, 8 % more.
+bool latencyBound(int chunks, int warps, double entriesPerRow) {
+    return 4LL * chunks <= 3LL * warps || (entriesPerRow > 16 && chunks <= 4LL * warps);
+}
 // Rows of an item where `rows` rows in all are shared by `warps` warps: whole
 // passes, so that every warp has some before any takes more than one pass.
 // Measured with the most rows throughout instead: 5 matrices of 100^2 to
@@ -114,8 +124,11 @@ __host__ __device__ constexpr int kVecOf() {
 // sides. A lane owns V consecutive right-hand sides of one row (R/V lanes per
 // row, 32V/R rows per pass) and runs one sequential fma chain per right-hand
 // side over the row's entries in CRS order. The rows' offsets are read once
-// per range by one coalesced load and passed around by shuffles.
-template <typename VT, typename XT, int R>
+// per range by one coalesced load and passed around by shuffles. U entries'
+// loads are in flight at a time: two where the L1 decides (four keep 13 % fewer
+// warps' x rows there: 254 and 281 us for the FP32 batch above), four where the
+// latency of a row does (kMpkBlock, FEW).
+template <typename VT, typename XT, int R, int U>
 __device__ __forceinline__ void blockRows(const BlockMember &m, int r0, int r1, int k) {
     constexpr int V = kVecOf<XT, R>();
     constexpr int L = R / V;        // lanes per row
@@ -139,9 +152,7 @@ __device__ __forceinline__ void blockRows(const BlockMember &m, int r0, int r1, 
             Vec acc;
 #pragma unroll
             for (int t = 0; t < V; ++t) acc.v[t] = XT(0);
-            // two entries at a time: four keep 13 % fewer warps' x rows in the L1
-            // (254 and 281 us for the FP32 batch above)
-#pragma unroll 2
+#pragma unroll U
             for (int e = e0; e < e1; ++e) {
                 const VT a = val[e];
                 const Vec xv = *reinterpret_cast<const Vec *>(xin + (size_t)col[e] * R);
@@ -154,8 +165,11 @@ __device__ __forceinline__ void blockRows(const BlockMember &m, int r0, int r1, 
 }
 
 // Relaxed polls, one acquire fence after the successful one (an acquire load
-// per flag empties the L1 each time) and a warp barrier behind the fence.
-template <typename VT, typename XT, int R>
+// per flag empties the L1 each time) and a warp barrier behind the fence. FEW
+// (few chunks, so that most items wait for their inputs and one latency follows
+// another): acquire loads, which unlike the fence do not wait for the warp's
+// own stores.
+template <typename VT, typename XT, int R, bool FEW>
 __global__ void __launch_bounds__(kBlockThreads) kMpkBlock(BlockArgs a) {
     const int lane = threadIdx.x & 31;
     for (;;) {
@@ -168,12 +182,13 @@ __global__ void __launch_bounds__(kBlockThreads) kMpkBlock(BlockArgs a) {
         const BlockMember m = a.members[h.z];
         if (k > 0) {
             const int *done = a.done + (size_t)(k - 1) * a.numChunks;
+            auto set = [&](int i) { return (FEW ? ldAcquireB(done + i) : ldRelaxedB(done + i)) != 0; };
             long long spins = 0;
             for (;;) {
                 bool ok = true;
-                for (int i = d0.x + lane; i <= d0.y; i += 32) ok &= ldRelaxedB(done + i) != 0;
-                for (int i = d0.z + lane; i <= d0.w; i += 32) ok &= ldRelaxedB(done + i) != 0;
-                for (int i = d1.x + lane; i <= d1.y; i += 32) ok &= ldRelaxedB(done + i) != 0;
+                for (int i = d0.x + lane; i <= d0.y; i += 32) ok &= set(i);
+                for (int i = d0.z + lane; i <= d0.w; i += 32) ok &= set(i);
+                for (int i = d1.x + lane; i <= d1.y; i += 32) ok &= set(i);
                 if (__all_sync(0xffffffffu, ok)) break;
                 if (++spins > kSpinLimit || ldAcquireB(a.status) != DEV_OK) {
                     if (lane == 0) atomicCAS(a.status, DEV_OK, DEV_WAIT_TIMEOUT);
@@ -181,10 +196,10 @@ __global__ void __launch_bounds__(kBlockThreads) kMpkBlock(BlockArgs a) {
                 }
                 __nanosleep(32);
             }
-            asm volatile("fence.acq_rel.gpu;" ::: "memory");
+            if (!FEW) asm volatile("fence.acq_rel.gpu;" ::: "memory");
             __syncwarp();  // a lane reads what other lanes' flags stand for; the vote orders nothing
         }
-        for (int r = h.x; r < h.y; r += 32) blockRows<VT, XT, R>(m, r, min(h.y, r + 32), k);
+        for (int r = h.x; r < h.y; r += 32) blockRows<VT, XT, R, FEW ? 4 : 2>(m, r, min(h.y, r + 32), k);
         __syncwarp();
         if (lane == 0)
             asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(a.done + (size_t)k * a.numChunks + d1.z), "r"(1)
@@ -199,7 +214,7 @@ __global__ void __launch_bounds__(kBlockThreads) kSpmvBlock(BlockMember m, int k
     const int warps = gridDim.x * (blockDim.x >> 5);
     const int rowsPerWarp = 32;
     for (int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); (long long)w * rowsPerWarp < m.n; w += warps)
-        blockRows<VT, XT, R>(m, w * rowsPerWarp, min(m.n, (w + 1) * rowsPerWarp), k);
+        blockRows<VT, XT, R, 4>(m, w * rowsPerWarp, min(m.n, (w + 1) * rowsPerWarp), k);
 }
 
 template <typename K>
@@ -211,14 +226,15 @@ int residentBlocksOf(K kernel) {
     return sms * std::max(occ, 1);
 }
 
-template <typename VT, typename XT, int R>
+template <typename VT, typename XT, int R, bool FEW = false>
 int blockResident() {
-    static const int blocks = residentBlocksOf(kMpkBlock<VT, XT, R>);
+    static const int blocks = residentBlocksOf(kMpkBlock<VT, XT, R, FEW>);
     return blocks;
 }
 template <typename VT, typename XT, int R>
-void launchBlock(const BlockArgs &a, cudaStream_t s) {
-    kMpkBlock<VT, XT, R><<<blockResident<VT, XT, R>(), kBlockThreads, 0, s>>>(a);
+void launchBlock(const BlockArgs &a, bool few, cudaStream_t s) {
+    if (few) kMpkBlock<VT, XT, R, true><<<blockResident<VT, XT, R, true>(), kBlockThreads, 0, s>>>(a);
+    else kMpkBlock<VT, XT, R, false><<<blockResident<VT, XT, R>(), kBlockThreads, 0, s>>>(a);
 }
 
 template <typename VT, typename XT, int R>
@@ -252,7 +268,7 @@ void dispatch(int valType, int vecType, int nrhs, A &&...args) {
 
 template <typename VT, typename XT, int R>
 struct LaunchBlockFn {
-    static void run(const BlockArgs &a, cudaStream_t s) { launchBlock<VT, XT, R>(a, s); }
+    static void run(const BlockArgs &a, bool few, cudaStream_t s) { launchBlock<VT, XT, R>(a, few, s); }
 };
 template <typename VT, typename XT, int R>
 struct WarpsInFlightFn {
@@ -288,13 +304,14 @@ void buildBatchTables(BatchTables &t, const std::vector<const BlockPlan *> &plan
     t.nrhs = p0.nrhs;
     t.maxPower = 0;
     std::vector<BlockMember> mem;
-    long long rows = 0;
+    long long rows = 0, entries = 0;
     for (const BlockPlan *p : plans) {
         if (p->valType != t.valType || p->vecType != t.vecType || p->nrhs != t.nrhs)
             throw Error(RACE_ERR_INCOMPATIBILITY, "batch members differ in value type, vector type or nrhs");
         t.maxPower = std::max(t.maxPower, p->power);
         mem.push_back(BlockMember{p->ops.rowPtr, p->ops.col, p->ops.val, p->ops.x, p->n, p->power});
         rows += p->n;
+        entries += p->entries;
     }
     // A batch's chunks: consecutive chunks of a member's plan and level group
     // put together up to the rows that the whole batch leaves each warp.
@@ -333,6 +350,7 @@ void buildBatchTables(BatchTables &t, const std::vector<const BlockPlan *> &plan
     // items by c + k lag (a lag of all chunks already is power by power);
     // twice the warps in flight: 281 us instead of 287 us at once that many
     const int lag = std::max(1, std::min(base, std::max(reach + 1, 2 * warps)));
+    t.few = latencyBound(base, warps, entries / (double)std::max<long long>(rows, 1));
     std::vector<int4> item;
     size_t total = 0;
     for (const Chunk &u : chunks) total += plans[u.member]->power;
@@ -385,6 +403,7 @@ std::unique_ptr<BlockPlan> buildBlockPlan(Engine &e, const race_operands &ops, i
     const int C = (int)chunkGroup.size();
     plan->numChunks = C;
     plan->chunkGroup = chunkGroup;
+    plan->entries = e.nnz;
     if (!chunkDependencyRanges(ops.rowPtr, ops.col, plan->chunkRow, chunkGroup, plan->depRange, e.stream))
         throw Error(RACE_ERR_INVALID_ARG,
                     "MPK operand is not in the engine's level order (permute it with getPerm/getInvPerm)");
@@ -399,7 +418,7 @@ void runBatch(BatchTables &t, int *status, cudaStream_t s) {
     RACE_CUDA(cudaMemsetAsync(t.ticket.p, 0, sizeof(int), s));
     if (t.numItems == 0) return;
     BlockArgs a{t.members.p, t.item.p, t.numItems, t.numChunks, t.done.p, t.ticket.p, status};
-    dispatch<LaunchBlockFn>(t.valType, t.vecType, t.nrhs, a, s);
+    dispatch<LaunchBlockFn>(t.valType, t.vecType, t.nrhs, a, t.few, s);
     RACE_CUDA(cudaGetLastError());
 }
 

@@ -103,6 +103,7 @@ struct BlockMember {
 struct BatchTables {
     int valType = 0, vecType = 0, nrhs = 1, maxPower = 0;
     int numChunks = 0, numItems = 0, numMembers = 0;
+    bool few = false;  // few chunks for the warps in flight (kMpkBlock)
     DevBuf<BlockMember> members;
     DevBuf<int4> item;                             // 3 per item, in issue order (batch.cu BlockArgs)
     DevBuf<int> done;                              // maxPower * numChunks
@@ -117,6 +118,7 @@ struct BlockPlan {
     std::vector<int> chunkRow;   // numChunks+1
     std::vector<int> depRange;   // numChunks*6 (local chunk ids, empty range [0,-1])
     std::vector<int> chunkGroup; // numChunks: level group
+    long long entries = 0;       // of the matrix (the engine's graph)
     BatchTables tables;
 };
 
