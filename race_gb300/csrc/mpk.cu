@@ -758,9 +758,14 @@ __device__ __forceinline__ void hubBlock(const SellView &m, int h, const float *
 //
 // kSpmvSell: a grid of resident warps striding the chunks, for matrices of
 // several chunks a warp, where loads in flight (occupancy) decide: FP32 runs
-// with 32 registers and 8 blocks an SM. Odd powers run from the last chunk to
-// the first: what the L2 still holds of a matrix that does not fit is its end
-// (27-point 97x113x89, FP32: 162 MB a power, 305 us with all powers forward).
+// with 32 registers and 8 blocks an SM. A chunk belongs to the same warp at
+// every power, and the next power's blocks start when this one's have ended,
+// on the same SMs: each die's L2 then holds the chunks of its own SMs. A warp
+// runs its chunks backwards at odd powers: what the L2 still holds of a matrix
+// that does not fit are the last ones. Measured, p = 8, launch by launch without
+// overlap / next blocks started early, other warps' chunks backwards / now:
+// 27-point 70^3 FP64 182 / 187 / 180 us, 80^3 281 / 263 / 234, 100^3 464 / 452 /
+// 433, FP32 351 / 268 / 253; 7-point 110^3 BF16 127 / 139 / 117.
 // Hub rows (FP64: their segments) come first, a warp each (STRIDE_HUBS), or,
 // where a row of some thousand entries lasts as long as a warp's chunks, to
 // warps that take nothing else (STRIDE_APART). Entries three at a time, to stay
@@ -771,7 +776,6 @@ template <typename VT, int FORM, bool C16>
 __global__ void __launch_bounds__(kWarpThreads, kSpmvMinBlocks<VT>)
     kSpmvSell(SellView m, HubWork hw, int numChunks, int n, int k, double *x, float *xf) {
     using AT = typename std::conditional<sizeof(VT) == 8, double, float>::type;
-    pdlTrigger();
     pdlWait();
     const int nw = gridDim.x * (blockDim.x >> 5), hubs = FORM == STRIDE ? 0 : hw.big + hw.num;
     int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), step = nw;
@@ -781,18 +785,18 @@ __global__ void __launch_bounds__(kWarpThreads, kSpmvMinBlocks<VT>)
         else xin = xf + (size_t)k * n;
         hubTask<VT, AT, 3>(m, hw, h - hw.big, k, n, xin, x, xf);
     };
+    if constexpr (FORM == STRIDE_HUBS)
+        for (; i < hubs; i += nw) hubRow(i);
     if constexpr (FORM == STRIDE_APART) {
         if (i < hubs) return hubRow(i);
         step = nw - hubs;
     }
-    for (; i < hubs + numChunks; i += step) {
-        if (FORM == STRIDE_HUBS && i < hubs) {
-            hubRow(i);
-            continue;
-        }
-        const int c = i - hubs;
-        chunkRow<VT, false, C16>(m, k & 1 ? numChunks - 1 - c : c, k, n, x, xf, 0);
-    }
+    int c = i - hubs;  // the warp's first chunk, less than step
+    if (c >= numChunks) return;
+    if (k & 1)
+        for (c += (numChunks - 1 - c) / step * step; c >= 0; c -= step) chunkRow<VT, false, C16>(m, c, k, n, x, xf, 0);
+    else
+        for (; c < numChunks; c += step) chunkRow<VT, false, C16>(m, c, k, n, x, xf, 0);
 }
 
 // kSpmvSellSmall: one piece of work a warp, for matrices of at most
