@@ -512,8 +512,9 @@ __global__ void __launch_bounds__(kWarpThreads, kMpkMinBlocks) kMpk(MpkArgs a) {
 }
 
 // Programmatic dependent launch: the next kernel of the stream may start (its
-// part before its own pdlWait) once every block of this one has; pdlWait
-// returns when the kernels before this one are complete and visible.
+// part before its own pdlWait) once every block of this one has called
+// pdlTrigger or ended; pdlWait returns when the kernels before this one are
+// complete and visible.
 __device__ __forceinline__ void pdlTrigger() { asm volatile("griddepcontrol.launch_dependents;"); }
 __device__ __forceinline__ void pdlWait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -537,6 +538,7 @@ __device__ __forceinline__ AT sellRowAhead(const VT *__restrict__ val, long long
     }
     if (len > 4) cn = groupCols<C16, false>(col, coff + 128, b, 0);
     pdlWait();
+    pdlTrigger();
     gather(c, len, xv);
     for (int j = 0; j < len; j += 4) {
         AT vn[4] = {AT(0), AT(0), AT(0), AT(0)}, xn[4] = {AT(0), AT(0), AT(0), AT(0)};
@@ -602,6 +604,7 @@ __device__ __forceinline__ AT sellRowLate(const VT *__restrict__ val, const void
     }
     if (len > 4) cn = *(const uint2 *)(cols + 128);
     pdlWait();
+    pdlTrigger();
     gather(c, len, xv);
     for (int j = 0; j < len; j += 4) {
         AT v[4], xn[4] = {AT(0), AT(0), AT(0), AT(0)};
@@ -802,14 +805,17 @@ __global__ void __launch_bounds__(kWarpThreads, kSpmvMinBlocks<VT>)
 // kSpmvSellSmall: one piece of work a warp, for matrices of at most
 // kSmallWarpsPerSm chunks an SM and those with hub rows, where the chain of
 // loads of a single row decides: row tables and first entry groups are read
-// before the previous power is complete, later groups ahead of their chain
-// (7-point 32^3: 13.7 us with only the matrix ahead, 11.9 us with x ahead too),
-// hub rows with eight gathers a lane in flight.
+// before the previous power is complete, later groups ahead of their chain, hub
+// rows with eight gathers a lane in flight. The next power's blocks may start
+// when this one's have their input. Started with this one's, blocks of several
+// powers crowd on the SMs that are free first (7-point 32^3 FP64, p = 4, 13.7
+// and 8.6 us; 27-point 30^3, p = 8, 70 and 37). FP32 and BF16 hub rows want
+// their blocks there as early as may be (150k-row power-law graph 107 and 112).
 template <typename VT, bool HUBS, bool C16>
 __global__ void __launch_bounds__(kWarpThreads, kSmallWarpsPerSm * 32 / kWarpThreads)
     kSpmvSellSmall(SellView m, HubWork hw, int numChunks, int n, int k, double *x, float *xf) {
     using AT = typename std::conditional<sizeof(VT) == 8, double, float>::type;
-    pdlTrigger();
+    if constexpr (HUBS && sizeof(VT) != 8) pdlTrigger();
     const AT *xin;
     if constexpr (sizeof(VT) == 8) xin = x + (size_t)k * n;
     else xin = xf + (size_t)k * n;
@@ -824,6 +830,7 @@ __global__ void __launch_bounds__(kWarpThreads, kSmallWarpsPerSm * 32 / kWarpThr
         }
         if (c < hw.num) {
             pdlWait();
+            pdlTrigger();
             hubTask<VT, AT, 8>(m, hw, c, k, n, xin, x, xf);
             return;
         }
