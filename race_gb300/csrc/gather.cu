@@ -125,8 +125,9 @@ __global__ void __launch_bounds__(kGatherThreads) kGatherLong(GatherArgs a) {
             [&](int k) {
                 const int p = a.entry[k0 + k];
                 if (p >= 0) return Pair<XT>{ld<VT, XT>(val, p), x[a.src[k0 + k]], false};
-                // the row's own update; a row without entries has none
-                return e > s ? Pair<XT>{ld<VT, XT>(val, s), x[y], true} : Pair<XT>{XT(0), XT(0), false};
+                // the row's own update; a row without entries has none (adding -0
+                // keeps a -0 as well)
+                return e > s ? Pair<XT>{ld<VT, XT>(val, s), x[y], true} : Pair<XT>{XT(-0.0), XT(0), false};
             },
             [&](XT v, XT xv, bool own) {
                 acc = mac(v, xv, acc);
