@@ -222,9 +222,9 @@ int race_spmv_power_layout(race_engine *e, int func_id, int k);
  * a stored column index (16: a 2-bit window and a 14-bit offset from one of
  * the chunk's four window bases; 32: plain indices), the chunks that keep
  * 32-bit columns in the 16-bit layout, the SELL slots with padding, and the
- * bytes of the matrix arrays one power reads (values, columns, row lengths,
- * chunk tables, hub copies), and the schedule that runs (see
- * race_set_mpk_schedule). */
+ * bytes of the matrix arrays the powers read (values, columns, row lengths,
+ * chunk tables, hub copies, the FP32 copy of long FP32/BF16 hub rows' values),
+ * and the schedule that runs (see race_set_mpk_schedule). */
 int race_get_mpk_layout(race_engine *e, int func_id, int *numChunks, int *colBits, int *wideChunks,
                         long long *sellSlots, long long *matrixBytes, int *schedule);
 

@@ -470,7 +470,7 @@ int race_get_mpk_layout(race_engine *e, int func_id, int *numChunks, int *colBit
     *matrixBytes = p.sellSlots * vb + (p.col16 ? 2 * p.sellSlots + 4 * p.wideSlots + 16LL * p.numChunks
                                                 : 4 * p.sellSlots) +
                    4LL * (long long)p.rowLen.n + 12LL * p.numChunks + 4LL * (long long)p.hubRow.n +
-                   (vb + 4) * (long long)p.hubCol.n;
+                   (vb + 4) * (long long)p.hubCol.n + (p.hubBig ? 4LL * (long long)p.hubBigVal.n : 0);
     *schedule = p.schedule != RACE_MPK_AUTO ? p.schedule : p.chosen;
     return RACE_SUCCESS;
 }
