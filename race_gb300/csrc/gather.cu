@@ -398,19 +398,37 @@ void buildGather(Engine &e, FuncEntry &f, int dir, const std::vector<int> &rp, c
     const bool lists = f.kernel != RACE_K_SPMV, own = f.kernel != RACE_K_SPMTV;
     const int first = f.kernel == RACE_K_SYMMSPMV ? 1 : 0;
     cudaStream_t s = e.stream;
-    GatherPlan gp;
-    if (lists) gp = buildGatherPlan(f.kernel, n, rp.data(), cl.data(), e.phases[dir]);
-    std::vector<int> len, longY;
+    GatherOrder go;
+    if (lists) go = buildGatherOrder(f.kernel, n, rp.data(), cl.data(), e.phases[dir]);
+    const std::vector<int> &ptr = go.ptr;
+    auto spread = [&](const std::vector<int> &offsets) {  // shortest and longest
+        int lo = INT_MAX, hi = 0;
+        const int *p = offsets.data();
+        for (int y = 0; y < n; ++y) {
+            const int len = p[y + 1] - p[y];
+            lo = std::min(lo, len);
+            hi = std::max(hi, len);
+        }
+        return std::pair<int, int>(lo, hi);
+    };
+    const auto [shortRow, longRow] = own ? spread(rp) : std::pair<int, int>(1, 0);
+    const int longList = lists ? spread(ptr).second : 0, most = std::max(longRow - first, longList);
+    const long long entries = lists ? ptr[n] : 0;
+    const bool f64 = f.ops.vec_type == RACE_VAL_F64;
+    const double updates = ((own ? (double)rp[n] - first * (double)n : 0.0) + entries) / std::max(n, 1);
+    g.plain = most <= kLongList && gatherPlain(f.kernel, f64, n, updates);
+    // Short lists of rows that all have entries are laid out here, straight
+    // from the walk; the others on the GPU from the plain ones (kListLayout).
+    const bool direct = lists && !g.plain && most <= kLongList && !(first && shortRow == 0);
+    std::vector<int> len, longY, pos, src;
     std::vector<long long> listOff;
     long long listSlots = 0;
+    GatherPlan gp;
+    if (lists && !direct) gp = buildGatherPlan(go, n, rp.data(), cl.data());
     auto lens = [&](int y) {
-        return std::pair<int, int>(own ? std::max(0, rp[y + 1] - rp[y] - first) : 0, lists ? gp.ptr[y + 1] - gp.ptr[y] : 0);
+        return std::pair<int, int>(own ? std::max(0, rp[y + 1] - rp[y] - first) : 0, lists ? ptr[y + 1] - ptr[y] : 0);
     };
     auto cut = [&](int line) {
-        len.assign(std::max(n, 1), 0);
-        listOff.assign(std::max(C, 1), 0);
-        longY.clear();
-        listSlots = 0;
         for (int c = 0; c < C; ++c) {
             int width = 0;
             for (int y = 32 * c; y < std::min(n, 32 * c + 32); ++y) {
@@ -421,7 +439,7 @@ void buildGather(Engine &e, FuncEntry &f, int dir, const std::vector<int> &rp, c
                     continue;
                 }
                 if (first && rp[y] == rp[y + 1]) {  // its own update is left out (kListLayout)
-                    for (int i = gp.ptr[y]; i < gp.ptr[y + 1]; ++i) cnt -= gp.entry[i] < 0;
+                    for (int i = ptr[y]; i < ptr[y + 1]; ++i) cnt -= gp.entry[i] < 0;
                 }
                 len[y] = cnt;
                 width = std::max(width, cnt);
@@ -430,32 +448,50 @@ void buildGather(Engine &e, FuncEntry &f, int dir, const std::vector<int> &rp, c
             listSlots += 32LL * ((width + 3) & ~3);
         }
     };
-    const bool f64 = f.ops.vec_type == RACE_VAL_F64;
-    int most = 0;
-    for (int y = 0; own && y < n; ++y) most = std::max(most, rp[y + 1] - rp[y] - first);
-    for (int y = 0; lists && y < n; ++y) most = std::max(most, gp.ptr[y + 1] - gp.ptr[y]);
-    const double updates = ((own ? (double)rp[n] - first * (double)n : 0.0) + gp.entry.size()) / std::max(n, 1);
-    g.plain = most <= kLongList && gatherPlain(f.kernel, f64, n, updates);
-    if (!g.plain) {
-        const int line = most > kLongList ? foldLine(n, f64, lens) : kLongList;
-        cut(line);
+    if (direct) {
+        len.resize(n);
+        listOff.resize(C);
+        for (int c = 0; c < C; ++c) {
+            const int y0 = 32 * c, y1 = std::min(n, y0 + 32);
+            int width = 0;
+            for (int y = y0; y < y1; ++y) {
+                len[y] = ptr[y + 1] - ptr[y];
+                width = std::max(width, len[y]);
+            }
+            listOff[c] = listSlots;
+            listSlots += 32LL * ((width + 3) & ~3);
+        }
+        pos.resize(listSlots);
+        src.resize(listSlots);
+        std::vector<long long> next(n);
+        for (int y = 0; y < n; ++y) next[y] = listOff[y >> 5] + 4 * (y & 31);
+        go.updates(n, rp.data(), cl.data(), [&](int y, int entry, int row) {
+            const long long at = next[y];
+            pos[at] = entry >= 0 ? entry : (rp[y] | INT_MIN);
+            src[at] = row;
+            next[y] = at + ((at & 3) == 3 ? 32 * 4 - 3 : 1);  // groups of four per lane
+        });
+    } else if (!g.plain) {
+        len.assign(std::max(n, 1), 0);
+        listOff.assign(std::max(C, 1), 0);
+        cut(most > kLongList ? foldLine(n, f64, lens) : kLongList);
     }
     // the longest first: a warp each, and the longest bounds the launch
     auto work = [&](int y) {
-        return (lists ? gp.ptr[y + 1] - gp.ptr[y] : 0) + (own ? rp[y + 1] - rp[y] : 0);
+        return (lists ? ptr[y + 1] - ptr[y] : 0) + (own ? rp[y + 1] - rp[y] : 0);
     };
     std::stable_sort(longY.begin(), longY.end(), [&](int a, int b) { return work(a) > work(b); });
     g.numLong = (int)longY.size();
-    // one allocation for all tables (each costs a first call 30-60 us)
+    // one allocation for all tables (above a megabyte each costs a first call 90 us)
     size_t total = 0;
     auto room = [&](size_t count) {
         const size_t at = total;
         total += (count + 3) & ~(size_t)3;
         return at;
     };
-    const size_t entries = gp.entry.size();
+    const size_t plain = gp.entry.size();
     const size_t oOff = room(2 * listOff.size()), oLen = room(len.size()), oLong = room(longY.size()),
-                 oPtr = room(gp.ptr.size()), oEntry = room(entries), oRow = room(entries), oPos = room(listSlots),
+                 oPtr = room(gp.ptr.size()), oEntry = room(plain), oRow = room(plain), oPos = room(listSlots),
                  oSrc = room(listSlots);
     g.mem.alloc(total);
     g.listOff = (long long *)(g.mem.p + oOff);
@@ -471,11 +507,14 @@ void buildGather(Engine &e, FuncEntry &f, int dir, const std::vector<int> &rp, c
     };
     put(g.len, len.data(), sizeof(int) * len.size());
     put(g.longY, longY.data(), sizeof(int) * longY.size());
-    if (lists) {
+    put(g.listOff, listOff.data(), sizeof(long long) * listOff.size());
+    if (direct) {
+        put(g.listPos, pos.data(), sizeof(int) * pos.size());
+        put(g.listSrc, src.data(), sizeof(int) * src.size());
+    } else if (lists) {
         put(g.ptr, gp.ptr.data(), sizeof(int) * gp.ptr.size());
-        put(g.entry, gp.entry.data(), sizeof(int) * entries);
-        put(g.row, gp.row.data(), sizeof(int) * entries);
-        put(g.listOff, listOff.data(), sizeof(long long) * listOff.size());
+        put(g.entry, gp.entry.data(), sizeof(int) * plain);
+        put(g.row, gp.row.data(), sizeof(int) * plain);
         if (C > 0 && !g.plain)
             kListLayout<<<ceilDiv(32LL * C, 256), 256, 0, s>>>(n, C, g.len, g.ptr, g.entry, g.row, f.ops.rowPtr, g.listOff,
                                                                g.listPos, g.listSrc);

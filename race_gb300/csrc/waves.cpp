@@ -137,38 +137,37 @@ FlowOrder buildFlowOrder(int kernel, int n, const int *rowPtr, const int *col, c
     return fo;
 }
 
-GatherPlan buildGatherPlan(int kernel, int n, const int *rowPtr, const int *col, const PhaseTable &pt) {
-    GatherPlan gp;
-    if (kernel != RACE_K_SPMTV && kernel != RACE_K_SYMMSPMV) return gp;
-    const std::vector<int> order = executionOrder(n, pt);
-    // count, then fill the updates of every b entry in execution order
-    const bool symm = kernel == RACE_K_SYMMSPMV;
-    std::vector<int> count(n + 1, 0);
-    for (int r : order) {
-        const int first = symm ? rowPtr[r] + 1 : rowPtr[r];
-        if (symm) ++count[r + 1];
+GatherOrder buildGatherOrder(int kernel, int n, const int *rowPtr, const int *col, const PhaseTable &pt) {
+    GatherOrder go;
+    go.symm = kernel == RACE_K_SYMMSPMV;
+    go.order = executionOrder(n, pt);
+    go.ptr.assign(n + 1, 0);
+    for (int r : go.order) {
+        const int first = go.symm ? rowPtr[r] + 1 : rowPtr[r];
+        if (go.symm) ++go.ptr[r + 1];
         for (int j = first; j < rowPtr[r + 1]; ++j)
-            if (col[j] >= 0 && col[j] < n) ++count[col[j] + 1];
+            if (col[j] >= 0 && col[j] < n) ++go.ptr[col[j] + 1];
     }
-    for (int y = 0; y < n; ++y) count[y + 1] += count[y];
-    gp.ptr = count;
-    gp.entry.assign(count[n], 0);
-    gp.row.assign(count[n], 0);
-    std::vector<int> fill(count.begin(), count.end() - 1);
-    for (int r : order) {
-        const int first = symm ? rowPtr[r] + 1 : rowPtr[r];
-        if (symm) {
-            gp.entry[fill[r]] = -1;
-            gp.row[fill[r]++] = r;
-        }
-        for (int j = first; j < rowPtr[r + 1]; ++j) {
-            const int c = col[j];
-            if (c < 0 || c >= n) continue;
-            gp.entry[fill[c]] = j;
-            gp.row[fill[c]++] = r;
-        }
-    }
+    for (int y = 0; y < n; ++y) go.ptr[y + 1] += go.ptr[y];
+    return go;
+}
+
+GatherPlan buildGatherPlan(const GatherOrder &go, int n, const int *rowPtr, const int *col) {
+    GatherPlan gp;
+    gp.ptr = go.ptr;
+    gp.entry.assign(go.ptr[n], 0);
+    gp.row.assign(go.ptr[n], 0);
+    std::vector<int> fill(go.ptr.begin(), go.ptr.end() - 1);
+    go.updates(n, rowPtr, col, [&](int y, int entry, int row) {
+        gp.entry[fill[y]] = entry;
+        gp.row[fill[y]++] = row;
+    });
     return gp;
+}
+
+GatherPlan buildGatherPlan(int kernel, int n, const int *rowPtr, const int *col, const PhaseTable &pt) {
+    if (kernel != RACE_K_SPMTV && kernel != RACE_K_SYMMSPMV) return GatherPlan{};
+    return buildGatherPlan(buildGatherOrder(kernel, n, rowPtr, col, pt), n, rowPtr, col);
 }
 
 }  // namespace race

@@ -49,4 +49,23 @@ struct GatherPlan {
 
 GatherPlan buildGatherPlan(int kernel, int n, const int *rowPtr, const int *col, const PhaseTable &pt);
 
+// The same in two steps: the rows in execution order and the plan's offsets,
+// then the updates one by one.
+struct GatherOrder {
+    bool symm = false;
+    std::vector<int> order, ptr;
+    // put(entry of b, matrix entry or -1, source row) for every update
+    template <typename F>
+    void updates(int n, const int *rowPtr, const int *col, F &&put) const {
+        for (int r : order) {
+            if (symm) put(r, -1, r);
+            for (int j = symm ? rowPtr[r] + 1 : rowPtr[r]; j < rowPtr[r + 1]; ++j)
+                if (col[j] >= 0 && col[j] < n) put(col[j], j, r);
+        }
+    }
+};
+
+GatherOrder buildGatherOrder(int kernel, int n, const int *rowPtr, const int *col, const PhaseTable &pt);
+GatherPlan buildGatherPlan(const GatherOrder &go, int n, const int *rowPtr, const int *col);
+
 }  // namespace race
