@@ -33,7 +33,7 @@
 // right behind one another, so that most warps waited): 24 matrices of 100^2
 // to 500^2, 8 FP32 right-hand sides, 587 and 254 us; 16 of 100^2 to 700^2, 16
 // FP64 ones, 2,015 and 1,832 us, 94 % of the FP64 pipe's time (1.08 G fma at 2
-// a cycle and SM); one of about 120^2, 16 FP32 ones, 62 and 51 us.
+// a cycle and SM); one of about 120^2, 16 FP32 ones, 47 and 39 us.
 #include <algorithm>
 
 #include <cuda_bf16.h>

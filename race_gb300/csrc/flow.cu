@@ -36,10 +36,10 @@
 // barrier of 152 blocks is 1.25 us, the row data loaded after it the rest),
 // the leaf executor one serial row after another in each leaf. Forward +
 // backward sweeps, before and after: Gauss-Seidel, 27-point 40x44x41 (leaf
-// sums, 248 waves a direction), FP64 2450 and 692 us; Kaczmarz, 9-point
-// 211x197 (leaf sums, 181 waves) 1150 and 511 us; the refinement solve of a
-// 100k-row power-law graph (sequential sums, FP32, 24 refinements of two
-// sweeps of 315 waves) 100 and 19.6 ms.
+// sums, 248 waves a direction), FP64 2450-2500 and 698-701 us; Kaczmarz, 9-point
+// 211x197 (leaf sums, 181 waves) 1150-1170 and 504-508 us; the refinement solve
+// of a 100k-row power-law graph (sequential sums, FP32, 24 refinements of two
+// sweeps of 315 waves; several graphs) 83-128 and 17-22 ms.
 #include <algorithm>
 #include <climits>
 

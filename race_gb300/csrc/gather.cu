@@ -6,9 +6,10 @@
 // no grid barriers. SpMV has no updates of other rows: its thread sums its own
 // row.
 //
-// Layout. The lists are per 32 consecutive entries of b (a warp) in groups of
-// four updates per lane, so that a warp reads 512 contiguous bytes of matrix
-// positions and of source rows at a time. The matrix values are always the
+// Layout (large matrices with short rows have none: gatherPlain). The lists are
+// per 32 consecutive entries of b (a warp) in groups of four updates per lane,
+// so that a warp reads 512 contiguous bytes of matrix positions and of source
+// rows at a time. The matrix values are always the
 // caller's, in place (they may change between calls). A row's own SymmSpMV
 // update (its diagonal, then its off-diagonal sum) stands in the list as its
 // diagonal's position with the sign bit, so that every step is the same fma.

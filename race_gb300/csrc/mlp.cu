@@ -12,7 +12,7 @@
 // another (kWeightGrad), which writes the caller's copy as well. Loss and
 // gradients of 239 rows, on the GPU and per call: one kernel per product (16
 // launches) 146 and 222 us; forward and backward kernels that fetch the weights
-// tile by tile and 32 x 32 gradient tiles 33 and 77 us; now 18.5 and 47 us
+// tile by tile and 32 x 32 gradient tiles 33 and 77 us; now 18.5 and 44-51 us
 // (512 rows 83 -> 54, 4,096: 131 -> 100, 65,536: 1,179 -> 883). Outputs alone,
 // 239 rows: 14.4 -> 10.3 us.
 // Networks that do not fit in shared memory take the tiles (kForward: a block

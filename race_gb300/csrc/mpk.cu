@@ -61,16 +61,17 @@ constexpr int kWarpThreads = 256;
 constexpr int kHubRowLen = kMpkHubRowLen;
 // Resident blocks per SM that the plain SpMV is compiled for (0: unbounded;
 // FP64 takes 40 registers, 6 blocks), and the warps per SM up to which every
-// warp gets at most one chunk. Measured: FP32 27-point 97x113x89, p = 8, 308 us
-// with 8 blocks and a few spilled words, 333 us with 40 registers; FP64
-// 60x61x63, p = 4, 59 us so, 64 us bounded to 6 blocks (which spills), and 66
-// us on the one-chunk kernel at two chunks a warp.
+// warp gets at most one chunk. Measured before the chunks kept their warps and
+// SMs (kSpmvSell): FP32 27-point 97x113x89, p = 8, 308 us with 8 blocks and a few
+// spilled words, 333 us with 40 registers; FP64 60x61x63, p = 4, 59 us so, 64 us
+// bounded to 6 blocks (which spills), and 66 us on the one-chunk kernel at two
+// chunks a warp.
 template <typename VT>
 constexpr int kSpmvMinBlocks = sizeof(VT) == 8 ? 0 : 8;
 constexpr int kSmallWarpsPerSm = 32;
 // Hub rows of FP32/BF16 values above this length are summed by a block each
 // (two tiles at least). The longest row bounds a power-law matrix, so the line
-// hardly matters: 110 and 116 us at 1,024 and 4,096 for the graph below.
+// hardly matters: 110 and 116 us at 1,024 and 4,096 for a 150k-row graph, BF16.
 constexpr int kHubBlockLen = 1024;
 // Longest FP32/BF16 hub row that a warp of the striding kernel takes
 // (spmvForm).
@@ -752,12 +753,12 @@ __device__ __forceinline__ void hubBlock(const SellView &m, int h, const float *
 
 // Plain x_{k+1} = A x_k on the SELL layout, no schedule: one warp per chunk,
 // and per hub row or segment (they come first: the longest work). The next
-// power's launch overlaps this one's tail (pdlTrigger), which took 2-3 us a
-// power. Measured on GB300, before all of this and now: 7-point 32^3, FP64,
-// p = 4 (launches): 25.3 and 11.9 us; BF16, 150k-row power-law graph, p = 4: 790
-// us with one warp per hub row (rows of up to 80k entries), 112 us; 27-point
-// 97x113x89, FP32, p = 8: 350 and 252 us; 7-point 110x101x107, FP64, p = 4: 119
-// and 92 us.
+// power's launch overlaps this one's end (programmatic dependent launch), which
+// took 2-3 us a power. Measured on GB300 over several boxes and graphs, with
+// plain launches one behind another and a warp per chunk or hub row / now:
+// 7-point 32^3, FP64, p = 4: 25.3 / 8.3-9.3 us; BF16, 150k-row power-law graphs,
+// p = 4: 504-831 / 108-156 us; 27-point 97x113x89, FP32, p = 8: 350 / 256-257 us;
+// 7-point 110^3, FP64, p = 8: 247 / 198 us.
 //
 // kSpmvSell: a grid of resident warps striding the chunks, for matrices of
 // several chunks a warp, where loads in flight (occupancy) decide: FP32 runs

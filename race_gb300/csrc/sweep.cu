@@ -670,8 +670,13 @@ void launch(bool waveMode, SweepArgs &a, int maxWork, cudaStream_t s) {
 // the cheaper of the two by a cost model fitted to GB300 timings (3D
 // stencils and power-law graphs): a wave costs about 12 us (barrier plus one
 // row's latency), a leaf phase about 1.3 us plus 0.67 us per row of its
-// longest leaf. For Gauss-Seidel and Kaczmarz it picks whose sums the
-// dataflow executor computes.
+// longest leaf. For Gauss-Seidel and Kaczmarz it picks whose sums the dataflow
+// executor computes, which has neither cost: the rule stays as it is because
+// another choice gives other roundings. Of 64 such calls of 4k to 730k rows it
+// takes the faster list in 47; it loses most on Gauss-Seidel with few threads
+// (27-point 80^3, 64 threads, FP64: sequential sums 3,914 us, lane sums 1,484;
+// power-law graph of 5,000 rows 919 and 360) and on Kaczmarz (7-point 90^3, 64
+// threads, FP32: 3,000 and 1,223). race_set_sweep_mode asks for either.
 bool useWaveMode(const Engine &e, const FuncEntry &f, int dir) {
     if (e.sweepMode == SWEEP_WAVE) return f.waves[dir].numWaves > 0;
     if (e.sweepMode == SWEEP_LEAF) return false;
@@ -876,8 +881,9 @@ void runSweep(Engine &e, FuncEntry &f, bool rev) {
     e.noteWaits();
     // Gauss-Seidel and Kaczmarz: by dataflow, which replaces a grid barrier
     // per wave (or a leaf's serial walk per phase) by one L2 round trip per
-    // dependent row, with the same sums; faster at every size measured
-    // (4k rows to 100k, see flow.cu)
+    // dependent row, with the same sums; 1.03 to 10 times faster at the sizes
+    // measured (4k rows to 6.25M, see flow.cu), but for the lane sums of a
+    // 6.25M-row 5-point matrix in FP32 (7.4 and 6.1 ms)
     if (f.flow[dir].ok) {
         runFlow(e, f, dir, !waveMode);
         return;
