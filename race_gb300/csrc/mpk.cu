@@ -59,15 +59,16 @@ namespace race {
 constexpr int kWarpThreads = 256;
 // Rows longer than this are summed by a whole warp from a contiguous copy.
 constexpr int kHubRowLen = kMpkHubRowLen;
-// Resident blocks per SM that the plain SpMV is compiled for (0: unbounded;
-// FP64 takes 40 registers, 6 blocks), and the warps per SM up to which every
-// warp gets at most one chunk. Measured before the chunks kept their warps and
-// SMs (kSpmvSell): FP32 27-point 97x113x89, p = 8, 308 us with 8 blocks and a few
-// spilled words, 333 us with 40 registers; FP64 60x61x63, p = 4, 59 us so, 64 us
-// bounded to 6 blocks (which spills), and 66 us on the one-chunk kernel at two
-// chunks a warp.
+// Resident blocks per SM that the plain SpMV is compiled for, and the warps per
+// SM up to which every warp gets at most one chunk. FP64: 40 registers without
+// a spilled word; left to itself the compiler takes 48 and 5 blocks fit
+// (27-point 60x61x63, p = 4, 58 and 54 us; 70^3, p = 8, 177 and 160; 7-point
+// 150^3, p = 1, 71 and 66). FP32 and BF16: 32 registers and a few spilled words;
+// measured before the chunks kept their warps and SMs (kSpmvSell), FP32 27-point
+// 97x113x89, p = 8, 308 us with 8 blocks and 333 us with 40 registers. FP64
+// 60x61x63, then 59 us: 66 us on the one-chunk kernel at two chunks a warp.
 template <typename VT>
-constexpr int kSpmvMinBlocks = sizeof(VT) == 8 ? 0 : 8;
+constexpr int kSpmvMinBlocks = sizeof(VT) == 8 ? 6 : 8;
 constexpr int kSmallWarpsPerSm = 32;
 // Hub rows of FP32/BF16 values above this length are summed by a block each
 // (two tiles at least). The longest row bounds a power-law matrix, so the line
@@ -757,8 +758,8 @@ __device__ __forceinline__ void hubBlock(const SellView &m, int h, const float *
 // took 2-3 us a power. Measured on GB300 over several boxes and graphs, with
 // plain launches one behind another and a warp per chunk or hub row / now:
 // 7-point 32^3, FP64, p = 4: 25.3 / 8.3-9.3 us; BF16, 150k-row power-law graphs,
-// p = 4: 504-831 / 108-156 us; 27-point 97x113x89, FP32, p = 8: 350 / 256-257 us;
-// 7-point 110^3, FP64, p = 8: 247 / 198 us.
+// p = 4: 504-831 / 108-156 us; 27-point 97x113x89, FP32, p = 8: 350 / 247-257 us;
+// 7-point 110^3, FP64, p = 8: 247 / 185 us.
 //
 // kSpmvSell: a grid of resident warps striding the chunks, for matrices of
 // several chunks a warp, where loads in flight (occupancy) decide: FP32 runs
@@ -768,8 +769,8 @@ __device__ __forceinline__ void hubBlock(const SellView &m, int h, const float *
 // runs its chunks backwards at odd powers: what the L2 still holds of a matrix
 // that does not fit are the last ones. Measured, p = 8, launch by launch without
 // overlap / next blocks started early, other warps' chunks backwards / now:
-// 27-point 70^3 FP64 182 / 187 / 180 us, 80^3 281 / 263 / 234, 100^3 464 / 452 /
-// 433, FP32 351 / 268 / 253; 7-point 110^3 BF16 127 / 139 / 117.
+// 27-point 70^3 FP64 182 / 187 / 160 us, 80^3 281 / 263 / 235, 100^3 464 / 452 /
+// 421, FP32 351 / 268 / 251; 7-point 110^3 BF16 127 / 139 / 117-121.
 // Hub rows (FP64: their segments) come first, a warp each (STRIDE_HUBS), or,
 // where a row of some thousand entries lasts as long as a warp's chunks, to
 // warps that take nothing else (STRIDE_APART). Entries three at a time, to stay
@@ -797,10 +798,9 @@ __global__ void __launch_bounds__(kWarpThreads, kSpmvMinBlocks<VT>)
     }
     int c = i - hubs;  // the warp's first chunk, less than step
     if (c >= numChunks) return;
-    if (k & 1)
-        for (c += (numChunks - 1 - c) / step * step; c >= 0; c -= step) chunkRow<VT, false, C16>(m, c, k, n, x, xf, 0);
-    else
-        for (; c < numChunks; c += step) chunkRow<VT, false, C16>(m, c, k, n, x, xf, 0);
+    if (k & 1) c = (numChunks - 1 - c) % step;  // the warp's last chunk, counted from the end
+    for (; c < numChunks; c += step)
+        chunkRow<VT, false, C16>(m, k & 1 ? numChunks - 1 - c : c, k, n, x, xf, 0);
 }
 
 // kSpmvSellSmall: one piece of work a warp, for matrices of at most
